@@ -114,6 +114,16 @@ int launch_quantity_read(int precision, const DftRegionDev& r, const void* const
   return 1;
 }
 
+// the factors exp(-2 pi i f n) of nsamp samples for nfb frequencies
+__device__ __forceinline__ void flush_twiddles(double2* tw, const double* freqs, int nfb, double nbase, int nsamp) {
+  for (int e = threadIdx.x; e < nsamp * nfb; e += blockDim.x) {
+    const int m = e / nfb, f = e % nfb;
+    double sn, cs;
+    sincospi(2.0 * freqs[f] * (nbase + m), &sn, &cs);
+    tw[m * 8 + f] = make_double2(cs, -sn);
+  }
+}
+
 template <typename R>
 __global__ void __launch_bounds__(256) dft_flush_kernel(int phase, const DftRegionDev* __restrict__ regions,
                                                         long long total, const R* __restrict__ buf,
@@ -127,12 +137,7 @@ __global__ void __launch_bounds__(256) dft_flush_kernel(int phase, const DftRegi
   for (int f0 = 0; f0 < g.nf; f0 += 8) {
     const int nfb = min(8, g.nf - f0);
     __syncthreads();
-    for (int e = threadIdx.x; e < nsamp * nfb; e += blockDim.x) {
-      const int m = e / nfb, f = e % nfb;
-      double sn, cs;
-      sincospi(2.0 * g.freqs[f0 + f] * (nbase + m), &sn, &cs);
-      tw[m * 8 + f] = make_double2(cs, -sn);
-    }
+    flush_twiddles(tw, g.freqs + f0, nfb, nbase, nsamp);
     __syncthreads();
     if (q >= g.npts) continue;
     double re[8] = {0, 0, 0, 0, 0, 0, 0, 0}, im[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -158,6 +163,50 @@ __global__ void __launch_bounds__(256) dft_flush_kernel(int phase, const DftRegi
   }
 }
 
+// The same sums in the same order for small regions: a thread per point would
+// walk 64 dependent round trips on a few CTAs (40 us for a row of 317
+// points). Here a CTA's threads first load the samples of 32 points together,
+// then take one frequency of one point each.
+constexpr int kFlushPts = 32;
+
+template <typename R>
+__global__ void __launch_bounds__(256) dft_flush_small_kernel(int phase, const DftRegionDev* __restrict__ regions,
+                                                              long long total, const R* __restrict__ buf,
+                                                              const Control* __restrict__ ctrl, int nsamp) {
+  __shared__ double2 tw[kDftChunk * 8];
+  __shared__ R xs[kDftChunk][kFlushPts];
+  const DftRegionDev& g = regions[blockIdx.y];
+  const int pt = threadIdx.x % kFlushPts, part = threadIdx.x / kFlushPts;
+  const long long q = static_cast<long long>(blockIdx.x) * kFlushPts + pt;
+  if (static_cast<long long>(blockIdx.x) * kFlushPts >= g.npts || nsamp <= 0) return;  // block-uniform
+  const double nbase = static_cast<double>(ctrl->dft_base) + (phase == 0 ? 1.0 : 1.5);
+  R v[kDftChunk / 8];
+#pragma unroll
+  for (int u = 0; u < kDftChunk / 8; u++) {
+    const int m = part + 8 * u;
+    v[u] = m < nsamp && q < g.npts ? buf[static_cast<long long>(m) * total + g.pt_off + q] : R(0);
+  }
+#pragma unroll
+  for (int u = 0; u < kDftChunk / 8; u++) xs[part + 8 * u][pt] = v[u];
+  for (int f0 = 0; f0 < g.nf; f0 += 8) {
+    const int nfb = min(8, g.nf - f0);
+    __syncthreads();
+    flush_twiddles(tw, g.freqs + f0, nfb, nbase, nsamp);
+    __syncthreads();
+    if (part >= nfb || q >= g.npts) continue;
+    double re = 0.0, im = 0.0;
+    for (int m = 0; m < nsamp; m++) {
+      const double x = static_cast<double>(xs[m][pt]) * g.acc_scale;
+      const double2 w = tw[m * 8 + part];
+      re += x * w.x;
+      im += x * w.y;
+    }
+    double* acc = g.acc + (static_cast<long long>(f0 + part) * g.npts + q) * 2;
+    acc[0] += re;
+    acc[1] += im;
+  }
+}
+
 // after a flush of nsamp samples the next sample is nsamp steps later
 __global__ void dft_rebase_kernel(Control* ctrl, int nsamp) { ctrl->dft_base += nsamp; }
 
@@ -179,11 +228,19 @@ int launch_dft_gather(int precision, const DftRegionDev* regions, int nreg, long
 int launch_dft_flush(int phase, int precision, const DftRegionDev* regions, int nreg, long long max_pts,
                      long long total_pts, const void* buf, const Control* ctrl, int nsamp, cudaStream_t s) {
   if (nreg == 0 || total_pts == 0 || nsamp <= 0) return 0;
-  dim3 grid(static_cast<unsigned>((max_pts + 255) / 256), nreg);
-  if (precision == 0)
-    dft_flush_kernel<double><<<grid, 256, 0, s>>>(phase, regions, total_pts, static_cast<const double*>(buf), ctrl, nsamp);
-  else
-    dft_flush_kernel<float><<<grid, 256, 0, s>>>(phase, regions, total_pts, static_cast<const float*>(buf), ctrl, nsamp);
+  const double* bd = static_cast<const double*>(buf);
+  const float* bf = static_cast<const float*>(buf);
+  // a thread per point once that fills the SMs (every load coalesced over 256
+  // points, each sample read once for all frequencies)
+  if ((max_pts + 255) / 256 * nreg < 148) {
+    const dim3 grid(static_cast<unsigned>((max_pts + kFlushPts - 1) / kFlushPts), nreg);
+    if (precision == 0) dft_flush_small_kernel<double><<<grid, 256, 0, s>>>(phase, regions, total_pts, bd, ctrl, nsamp);
+    else dft_flush_small_kernel<float><<<grid, 256, 0, s>>>(phase, regions, total_pts, bf, ctrl, nsamp);
+    return 1;
+  }
+  const dim3 grid(static_cast<unsigned>((max_pts + 255) / 256), nreg);
+  if (precision == 0) dft_flush_kernel<double><<<grid, 256, 0, s>>>(phase, regions, total_pts, bd, ctrl, nsamp);
+  else dft_flush_kernel<float><<<grid, 256, 0, s>>>(phase, regions, total_pts, bf, ctrl, nsamp);
   return 1;
 }
 
