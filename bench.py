@@ -93,7 +93,7 @@ def parse():
                     help="batch64: autotune, or force a launch mode (with --batch-rows)")
     ap.add_argument("--batch-rows", type=int, default=4, choices=[1, 2, 4, 8])
     ap.add_argument("--batch-temporal", type=int, default=0, choices=[0, 2, 3, 4],
-                    help="batch64 with a forced launch mode: steps per launch of temporal blocking (0: off)")
+                    help="batch64 with a forced launch mode: depth of temporal blocking (0: off)")
     ap.add_argument("--decompose", default="replicas", choices=["replicas", "zslab"],
                     help="single-grid workloads on N GPUs: independent replicas (weak scaling), or one grid cut "
                          "into z slabs, one per rank, ghost planes over NCCL overlapped with the interior sweep "
@@ -651,12 +651,12 @@ def run_batch(args, torch, world, rank, local, stream):
                    "interior_cells": total_cells, "seed": 0, "shard_imbalance": imbalance(
                        [problem_cost(p) for p in allp], shares),
                    "cpml": 10, "steps_in_config": 3000, "tile_rows": info["rows"], "ctas": info["blocks"],
-                   "launch": f"temporal blocking, {tb} steps per launch" if tb else info["launch"],
+                   "launch": f"temporal blocking, up to {2 * tb} steps per launch" if tb else info["launch"],
                    "tune_ms_per_step": info["tune_ms_per_step"],
                    "temporal_depth": tb, "tune_ms_per_step_temporal": tbi["tune_ms_per_step"],
                    "size_classes": classes, "tuned_ms_per_step": ir["tuned_ms_per_step"],
                    "l2": "state ~290 MB > L2; no flush", "parallelism": f"problems sharded by cost over {world} GPUs" if world > 1 else "single GPU"},
-        "roofline": {"bound": "hbm", "kernel": (f"batch_tb_kernel ({tb} steps per launch from shared memory; the "
+        "roofline": {"bound": "hbm", "kernel": (f"window_batch_kernel (up to {2 * tb} steps per launch in windows held on chip; the "
                                                 "fraction counts the one-sweep bytes of every step and can exceed 1)"
                                                 if tb else "batch_kernel (persistent, all steps)"
                                                 if info["launch"] == "persistent"

@@ -32,11 +32,12 @@ SOURCES = {
     "kernels_fused3d_async.cu": [],
     "kernels_tfsf.cu": [],
     "kernels_batch.cu": [],
+    "kernels_window.cu": [],
     "kernels_common.cu": [],
     "kernels_adjoint.cu": [],
     "fdtd_capi.cu": [],
 }
-HEADERS = ["internal.h", "fused3d_common.cuh", os.path.join("..", "..", "include", "fdtd_b200.h")]
+HEADERS = ["internal.h", "fused3d_common.cuh", "pairs.cuh", os.path.join("..", "..", "include", "fdtd_b200.h")]
 
 
 def _newer(target: str, deps) -> bool:

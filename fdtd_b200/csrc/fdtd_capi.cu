@@ -215,6 +215,13 @@ struct fdtd_grid {
   int scheme = 1;     // time policy of the curl updates: 1 BD1, 3 BD3, 4 BD4
   void* hist[2][3][3]{};  // FP64 flux history [D|B][level][comp] of BD3/BD4
   int sweep_kind = FDTD_SWEEP_AUTO;
+  // temporal blocking of 2D FP32 grids: the second copy of the state (fields,
+  // CPML integrators, soft sources' last values) and 1/eps per cell, the
+  // kernel's arguments and the version they were made for
+  void* win_block = nullptr;  // one allocation for all of it
+  WinArgs win{};
+  long long win_version = -1;
+  bool win_ok = false;
   TmaState* tma = nullptr;
   unsigned* d_eh = nullptr;  // one-launch step: [0] epoch, then the E tile flags
   long long eh_words = 0;
@@ -791,6 +798,168 @@ FusedArgs fused_args(fdtd_grid* g) {
   return a;
 }
 
+// ---- temporal blocking of 2D FP32 grids (kernels_window.cu)
+
+// The state arrays a window holds: fields and CPML integrators
+void window_arrays(const fdtd_grid* g, void* (&f)[3], void* (&psi)[4]) {
+  const bool te = g->d.mode == kTE;
+  f[0] = te ? g->E[0] : g->E[2];
+  f[1] = te ? g->E[1] : g->H[0];
+  f[2] = te ? g->H[2] : g->H[1];
+  psi[0] = g->psi[0][te ? 0 : 2][1];
+  psi[1] = g->psi[0][te ? 1 : 2][0];
+  psi[2] = g->psi[1][te ? 2 : 0][1];
+  psi[3] = g->psi[1][te ? 2 : 1][0];
+}
+
+// What the windows do not cover keeps the launches per half step: poles,
+// mu_r, TFSF planes, boundary conditions, DFT of surface quantities, more
+// boxes or regions than a window lists, and a sweep kernel set by hand.
+bool window_wanted(const fdtd_grid* g) {
+  if (!g->f32 || g->d.mode == kThreeD || g->sweep_kind != FDTD_SWEEP_AUTO) return false;
+  if (g->max_poles != 0 || g->bcs.n > 0 || !g->planes.empty()) return false;
+  if (g->boxes.size() > static_cast<size_t>(kWinMaxBoxes)) return false;
+  for (const auto& m : g->mats)
+    if (m.mu_r != 1.0) return false;
+  int n[2] = {0, 0};
+  for (const auto& r : g->dfts) {
+    if (r.comp >= 6) return false;
+    n[quantity_phase(r.comp)]++;
+  }
+  return n[0] <= kWinMaxRegions && n[1] <= kWinMaxRegions;
+}
+
+// The kernel's arguments but for the second copy of the state and 1/eps
+WinArgs window_args(fdtd_grid* g) {
+  const FusedArgs fa = fused_args(g);
+  WinArgs a;
+  memset(&a, 0, sizeof(a));
+  a.nx = fa.nx;
+  a.ny = fa.ny;
+  a.pitch = fa.pitch;
+  for (int x = 0; x < 2; x++) {
+    a.pml[x] = fa.pml_axis[x];
+    a.slab[x] = fa.slab[x];
+    for (int h = 0; h < 2; h++) a.prof[h][x] = fa.prof[h][x];
+    auto is_plain = [&](int i) {
+      return g->prof[0][x].F[i] == 1.0 && g->prof[1][x].F[i] == 1.0 && (!a.pml[x] || slab_index(a.slab[x], i) < 0);
+    };
+    int lo = g->n[x] / 2, hi = lo;
+    a.plain[x][0] = 1;
+    a.plain[x][1] = 0;
+    if (lo < 1 || lo > g->n[x] - 2 || !is_plain(lo)) continue;
+    while (lo > 1 && is_plain(lo - 1)) lo--;
+    while (hi < g->n[x] - 2 && is_plain(hi + 1)) hi++;
+    a.plain[x][0] = lo;
+    a.plain[x][1] = hi;
+  }
+  void *f[3], *psi[4];
+  window_arrays(g, f, psi);
+  for (int q = 0; q < 3; q++) a.f[0][q] = static_cast<float*>(f[q]);
+  for (int q = 0; q < 4; q++) a.psi[0][q] = static_cast<float*>(psi[q]);
+  a.src_last[0] = g->d_src_last;
+  a.src_scale_d = fa.src_scale_d;
+  a.src_scale_b = fa.src_scale_b;
+  a.src_scale_h = fa.src_scale_h;
+  a.eta = fa.eta;
+  a.nsrc = fa.nsrc;
+  for (int q = 0; q < fa.nsrc; q++) a.src[q] = fa.src[q];
+  a.nbox = static_cast<int>(std::min<size_t>(g->boxes.size(), kWinMaxBoxes));
+  for (int q = 0; q < a.nbox; q++) {
+    const BoxSourceH& b = g->boxes[q];
+    a.box[q] = WinBox{b.comp, b.target, {b.lo[0], b.lo[1]}, {b.hi[0], b.hi[1]}, b.nvals, b.d_vals};
+  }
+  for (int ph = 0; ph < 2; ph++) {
+    a.nreg[ph] = g->ndft[ph];
+    a.reg[ph] = g->d_dft[ph];
+    a.dft_buf[ph] = static_cast<float*>(g->d_dft_buf[ph]);
+    a.dft_pts[ph] = g->dft_pts[ph];
+  }
+  a.ctrl = g->ctrl;
+  // one material and no map: 1/eps is a constant
+  const bool uniform = !g->d_eps_map && ((!g->d_ids && !g->d_bids) || g->mats.size() == 1);
+  a.ie0 = uniform ? static_cast<float>(g->mats[0].kind == FDTD_VACUUM ? 1.0 : 1.0 / g->mats[0].eps_inf) : 0.f;
+  return a;
+}
+
+bool window_uniform(const fdtd_grid* g) {
+  return !g->d_eps_map && ((!g->d_ids && !g->d_bids) || g->mats.size() == 1);
+}
+
+// Lays out the second copy of the state and 1/eps of a grid that takes its
+// steps in windows, again after any change to it. A grid whose second copy
+// does not fit in device memory keeps the launches per half step.
+int ensure_window(fdtd_grid* g) {
+  if (g->win_version == g->version) return FDTD_OK;
+  g->win_ok = false;
+  if (!window_wanted(g)) {
+    g->win_version = g->version;
+    return FDTD_OK;
+  }
+  void *f[3], *psi[4];
+  window_arrays(g, f, psi);
+  // the parts of the block: fields, integrators, src_last, 1/eps
+  void* own[8] = {f[0], f[1], f[2], psi[0], psi[1], psi[2], psi[3], g->d_src_last};
+  size_t at[9], total = 0;
+  auto part = [&](int q, size_t bytes) {
+    at[q] = total;
+    total += (bytes + 255) / 256 * 256;
+  };
+  for (int q = 0; q < 8; q++) part(q, own[q] ? g->sizes[own[q]] : 0);
+  part(8, window_uniform(g) ? 0 : static_cast<size_t>(field_elems(g)) * sizeof(float));
+  if (!g->win_block || g->sizes[g->win_block] != total) {
+    dfree(g, g->win_block);
+    const int rc = dalloc(g, &g->win_block, total);
+    if (rc) {
+      g->win_version = g->version;
+      return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
+    }
+  }
+  g->win = window_args(g);
+  char* const b = static_cast<char*>(g->win_block);
+  for (int q = 0; q < 3; q++) g->win.f[1][q] = reinterpret_cast<float*>(b + at[q]);
+  for (int q = 0; q < 4; q++)
+    if (psi[q]) g->win.psi[1][q] = reinterpret_cast<float*>(b + at[3 + q]);
+  if (g->d_src_last) g->win.src_last[1] = reinterpret_cast<double*>(b + at[7]);
+  if (!window_uniform(g)) {
+    float* const ie = reinterpret_cast<float*>(b + at[8]);
+    g->win.ie = ie;
+    g->launches += launch_adjoint_inv_eps(fused_args(g), ie, g->stream);
+  }
+  // the windows read what was set up here before they wait for the launch
+  // ahead of them (launch_chained): it is all in place once this returns
+  CK(cudaStreamSynchronize(g->stream));
+  g->win_version = g->version;
+  g->win_ok = true;
+  return FDTD_OK;
+}
+
+// Steps per launch and rows per window: the pair with the least modelled time
+// of a step. A launch takes from its predecessor's end about 4 us + 1.05 us a
+// step with windows of 32 rows, 8 us + 1.5 us a step with 64 (measured at
+// 317 x 233), and each further round of windows (two per SM) 5 and 11.5 us +
+// 0.1 us a step (3001 x 2047: 32 rows 19.7 us a step at 8 steps, 64 rows 20.9
+// at 4, 14.3 at 8, 14.2 at 12, 16.3 at 16).
+int window_steps(int nx, int ny, int* rows) {
+  int best = 8;
+  double least = 1e30;
+  for (int R : {32, 64})
+    for (int L : {16, 12, 8, 6, 4}) {
+      const int T = (kGraphSteps + L - 1) / L;
+      if (4 * T > R + 16) continue;
+      const double rounds = window_count(nx, ny, R, T) / 296.0;
+      const double one = R == 32 ? 4.0 + 1.05 * T : 8.0 + 1.5 * T;
+      const double more = (R == 32 ? 5.0 : 11.5) + 0.1 * T;
+      const double t = (one + std::max(0.0, rounds - 1.0) * more) * L;
+      if (t < least) {
+        least = t;
+        best = T;
+        *rows = R;
+      }
+    }
+  return best;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1345,6 +1514,7 @@ int fdtd_dft_read(fdtd_grid* g, int handle, double* out) try {
 
 static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof);
 static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof);
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s);
 
 // The TFSF aux tables for a call of nsteps steps: at least 257 rows, so that
 // calls of up to 256 steps keep them (and the step graph, whose launches hold
@@ -1373,7 +1543,7 @@ static int ensure_step_graph(fdtd_grid* g, cudaStream_t s) {
   }
   const long long before = g->launches;
   CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_steps(g, kGraphSteps, s, nullptr);
+  int rc = g->win_ok ? enqueue_windows(g, kGraphSteps, s) : enqueue_steps(g, kGraphSteps, s, nullptr);
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &graph);
   if (rc) return rc;
@@ -1406,6 +1576,8 @@ int fdtd_prepare(fdtd_grid* g) try {
   }
   // the step graph too (its capture launches nothing), so that the first
   // call of kGraphSteps or more steps replays it at once
+  rc = ensure_window(g);
+  if (rc) return rc;
   if (g->use_graphs && g->next_half == 0 && !g->half_split) {
     rc = ensure_aux_tables(g, kGraphSteps);
     if (rc) return rc;
@@ -1550,6 +1722,40 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
   return FDTD_OK;
 }
 
+// Enqueues nsteps steps of a grid that takes them in windows: an even number
+// of launches per stretch of steps (ending on the grid's own arrays), each
+// stretch within the DFT sample ring; a single step left over goes out as
+// launches per half step.
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s) {
+  const bool dft = !g->dfts.empty();
+  int rows = kWinRows;
+  const int T = window_steps(g->n[0], g->n[1], &rows);
+  for (int done = 0; done < nsteps;) {
+    const int n = std::min(nsteps - done, kDftChunk - (dft ? g->dft_pending : 0));
+    if (n == 1) {
+      const int rc = enqueue_steps(g, 1, s, nullptr);
+      if (rc) return rc;
+      done++;
+      continue;
+    }
+    const int L = 2 * ((n + 2 * T - 1) / (2 * T));
+    for (int q = 0; q < L; q++) {
+      const int at = static_cast<int>(static_cast<long long>(n) * q / L);
+      const int t = static_cast<int>(static_cast<long long>(n) * (q + 1) / L) - at;
+      g->launches += launch_window(g->d.mode, g->win, rows, t, at, q & 1, g->dft_pending + at, s);
+    }
+    g->launches += launch_steps_advance(g->ctrl, n, s);
+    if (dft) {
+      g->dft_pending += n;
+      if (g->dft_pending == kDftChunk) g->launches += flush_dft(g, s);
+    }
+    done += n;
+  }
+  if (g->dft_pending > 0) g->launches += flush_dft(g, s);
+  CK(cudaGetLastError());
+  return FDTD_OK;
+}
+
 static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
   if (!g) return fail(FDTD_ERR_INVALID, "null grid");
   if (g->next_half != 0 || g->half_split) return fail(FDTD_ERR_INVALID, "an E half step was taken without its H half");
@@ -1562,6 +1768,13 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     if (prc) return prc;
     prc = ensure_eh(g);
     if (prc) return prc;
+    if (g->dirty_dft) {
+      prc = rebuild_dft(g);
+      if (prc) return prc;
+      CK(cudaStreamSynchronize(g->stream));
+    }
+    prc = ensure_window(g);
+    if (prc) return prc;
   }
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
   if (s != g->stream) {
@@ -1571,11 +1784,6 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     CK(cudaEventRecord(ev, g->stream));
     CK(cudaStreamWaitEvent(s, ev, 0));
     CK(cudaEventDestroy(ev));
-  }
-  if (g->dirty_dft) {
-    int rc = rebuild_dft(g);
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(g->stream));
   }
   // TFSF: precompute the aux grids' Ez/Hy for this chunk of steps
   {
@@ -1605,7 +1813,7 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     }
   }
   if (done < nsteps) {
-    int rc = enqueue_steps(g, nsteps - done, s, prof);
+    int rc = g->win_ok && !prof ? enqueue_windows(g, nsteps - done, s) : enqueue_steps(g, nsteps - done, s, prof);
     if (rc) return rc;
   }
   CK(cudaGetLastError());
@@ -2101,13 +2309,12 @@ struct fdtd_batch {
   // measured ms per step: persistent with rows 1, 2, 4, 8, then per-phase with rows 1, 2, 4, 8
   std::vector<float> tune_ms;
   float tune_best_ms = 0.f;  // with the per-class item heights
-  // temporal blocking (fdtd_batch_set_temporal): steps per launch (0: off),
-  // the grids' arguments on the second copy of their state, the tiles
+  // temporal blocking (fdtd_batch_set_temporal): its depth (0: off; a launch
+  // takes up to 2 * depth steps), the windows' arguments and work lists
   int tb = 0;
-  FusedArgs* d_args_b = nullptr;
-  unsigned* d_tb_items = nullptr;
-  int n_tb_items = 0;
-  std::vector<void*> tb_bufs;  // the second copy
+  WinArgs* d_win = nullptr;
+  std::map<int, std::pair<unsigned*, int>> tb_items;  // the windows, by steps per launch
+  std::vector<void*> tb_bufs;  // the second copy of the state, 1/eps per cell
   std::vector<float> tb_ms;    // tuner: ms per step with 2, 3 and 4 steps per launch (0: not timed)
 };
 
@@ -2176,51 +2383,51 @@ const char* tb_unsupported(const fdtd_batch* b) {
   return nullptr;
 }
 
-// frees the second copy of the state and the tiles (temporal blocking off)
+// frees the second copy of the state and the work lists (temporal blocking off)
 void tb_release(fdtd_batch* b) {
-  cudaFree(b->d_args_b);
-  cudaFree(b->d_tb_items);
+  cudaFree(b->d_win);
+  for (auto& kv : b->tb_items) cudaFree(kv.second.first);
   for (void* p : b->tb_bufs) cudaFree(p);
-  b->d_args_b = nullptr;
-  b->d_tb_items = nullptr;
-  b->n_tb_items = 0;
+  b->d_win = nullptr;
+  b->tb_items.clear();
   b->tb_bufs.clear();
   b->tb = 0;
 }
 
 // The second copy of every array a step changes (fields, CPML integrators,
-// the soft sources' last values) and the grids' arguments pointing at it;
-// laid out once, a copy of the current state. On failure nothing is kept.
+// the soft sources' last values), 1/eps per cell and the windows' arguments;
+// laid out once. On failure nothing is kept.
 int tb_prepare(fdtd_batch* b) {
-  if (b->d_args_b) return FDTD_OK;
+  if (b->d_win) return FDTD_OK;
   CK(cudaDeviceSynchronize());
-  std::vector<FusedArgs> args = b->h_args;
+  std::vector<WinArgs> args;
   bool ok = true;
   for (size_t q = 0; q < b->grids.size() && ok; q++) {
     fdtd_grid* g = b->grids[q];
-    FusedArgs& a = args[q];
-    // a same-sized copy of the state array p (null if p is not one)
-    auto twin = [&](void* p) -> void* {
-      if (!g->sizes.count(p)) return nullptr;
+    WinArgs a = window_args(g);
+    auto room = [&](size_t bytes) -> void* {
       void* d = nullptr;
-      if (cudaMalloc(&d, g->sizes[p]) != cudaSuccess) return nullptr;
+      if (cudaMalloc(&d, bytes) != cudaSuccess) return nullptr;
       b->tb_bufs.push_back(d);
-      if (cudaMemcpy(d, p, g->sizes[p], cudaMemcpyDeviceToDevice) != cudaSuccess) return nullptr;
-      return d;
+      return cudaMemsetAsync(d, 0, bytes, g->stream) == cudaSuccess ? d : nullptr;
     };
-    for (int c = 0; c < 3 && ok; c++) {
-      if (g->E[c]) ok = ok && (a.E[c] = static_cast<float*>(twin(g->E[c])));
-      if (g->H[c]) ok = ok && (a.H[c] = static_cast<float*>(twin(g->H[c])));
+    // room for a copy of the state array p
+    auto twin = [&](void* p) -> void* { return g->sizes.count(p) ? room(g->sizes[p]) : nullptr; };
+    for (int c = 0; c < 3 && ok; c++) ok = (a.f[1][c] = static_cast<float*>(twin(a.f[0][c])));
+    for (int c = 0; c < 4 && ok; c++)
+      if (a.psi[0][c]) ok = (a.psi[1][c] = static_cast<float*>(twin(a.psi[0][c])));
+    if (ok && a.src_last[0]) ok = (a.src_last[1] = static_cast<double*>(twin(a.src_last[0])));
+    if (ok && !window_uniform(g)) {
+      float* ie = static_cast<float*>(room(static_cast<size_t>(field_elems(g)) * sizeof(float)));
+      if (ie) launch_adjoint_inv_eps(b->h_args[q], ie, g->stream);
+      ok = ie != nullptr;
+      a.ie = ie;
     }
-    for (int ft = 0; ft < 2; ft++)
-      for (int I = 0; I < 3; I++)
-        for (int J = 0; J < 3; J++)
-          if (g->psi[ft][I][J]) ok = ok && (a.psi[ft][I][J] = static_cast<float*>(twin(g->psi[ft][I][J])));
-    if (g->d_src_last) ok = ok && (a.src_last = static_cast<double*>(twin(g->d_src_last)));
+    args.push_back(a);
   }
-  if (ok) ok = cudaMalloc(&b->d_args_b, args.size() * sizeof(FusedArgs)) == cudaSuccess;
-  if (ok)
-    ok = cudaMemcpy(b->d_args_b, args.data(), args.size() * sizeof(FusedArgs), cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) ok = cudaMalloc(&b->d_win, args.size() * sizeof(WinArgs)) == cudaSuccess;
+  if (ok) ok = cudaMemcpy(b->d_win, args.data(), args.size() * sizeof(WinArgs), cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) ok = cudaDeviceSynchronize() == cudaSuccess;
   if (!ok) {
     const cudaError_t e = cudaGetLastError();
     tb_release(b);
@@ -2229,40 +2436,56 @@ int tb_prepare(fdtd_batch* b) {
   return FDTD_OK;
 }
 
-// the tiles of the temporally blocked launches of depth `depth`
-int tb_items(fdtd_batch* b, int depth) {
-  int tw = 0, th = 0;
-  if (!batch_tb_tile(depth, &tw, &th)) return fail(FDTD_ERR_INVALID, "temporal blocking depth must be 2, 3 or 4");
+// the windows of launches of T steps
+int tb_windows(fdtd_batch* b, int T) {
+  if (b->tb_items.count(T)) return FDTD_OK;
   std::vector<unsigned> items;
   for (size_t q = 0; q < b->grids.size(); q++) {
     const fdtd_grid* g = b->grids[q];
-    const long long nt = static_cast<long long>((g->n[0] + tw - 1) / tw) * ((g->n[1] + th - 1) / th);
+    const int nt = window_count(g->n[0], g->n[1], kWinRows, T);
     if (nt >= (1 << 24)) return fail(FDTD_ERR_UNSUPPORTED, "grid too large to batch");
-    for (long long t = 0; t < nt; t++) items.push_back(static_cast<unsigned>(q) << 24 | static_cast<unsigned>(t));
+    for (int t = 0; t < nt; t++) items.push_back(static_cast<unsigned>(q) << 24 | static_cast<unsigned>(t));
   }
-  if (b->d_tb_items) cudaFree(b->d_tb_items);
-  b->d_tb_items = nullptr;
-  b->n_tb_items = static_cast<int>(items.size());
-  CK(cudaMalloc(&b->d_tb_items, items.size() * sizeof(unsigned)));
-  CK(cudaMemcpy(b->d_tb_items, items.data(), items.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+  unsigned* d = nullptr;
+  CK(cudaMalloc(&d, items.size() * sizeof(unsigned)));
+  b->tb_items[T] = {d, static_cast<int>(items.size())};
+  CK(cudaMemcpy(d, items.data(), items.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+  return FDTD_OK;
+}
+
+// The steps of each launch of a call of nsteps steps with temporal blocking:
+// an even number of launches (there and back, so that the state ends in the
+// grids' own arrays) of at most 2 * depth steps each, as equal as they come;
+// none for a single step, which goes out as launches per half step.
+std::vector<int> tb_schedule(const fdtd_batch* b, int nsteps) {
+  std::vector<int> out;
+  if (b->tb <= 0 || nsteps < 2) return out;
+  const int T = 2 * b->tb, L = 2 * ((nsteps + 2 * T - 1) / (2 * T));
+  for (int q = 0; q < L; q++)
+    out.push_back(static_cast<int>(static_cast<long long>(nsteps) * (q + 1) / L - static_cast<long long>(nsteps) * q / L));
+  return out;
+}
+
+// the work lists that a call of nsteps steps needs (before any capture)
+int tb_ready(fdtd_batch* b, int nsteps) {
+  for (int T : tb_schedule(b, nsteps)) {
+    const int rc = tb_windows(b, T);
+    if (rc) return rc;
+  }
   return FDTD_OK;
 }
 
 int batch_launch(fdtd_batch* b, int nsteps, cudaStream_t s) {
   const FusedArgs* args = b->d_args;
   const unsigned* items = b->d_items;
-  int s0 = 0;
-  if (b->tb > 0) {
-    // pairs of launches of tb steps each, there and back, so that the state
-    // ends in the grids' own arrays; the rest one kernel per half step
-    const int T = b->tb, pairs = nsteps / (2 * T);
-    for (int p = 0; p < pairs; p++) {
-      launch_batch_tb(b->mode, T, b->d_args, b->d_args_b, b->d_tb_items, b->n_tb_items, s0, s);
-      launch_batch_tb(b->mode, T, b->d_args_b, b->d_args, b->d_tb_items, b->n_tb_items, s0 + T, s);
-      s0 += 2 * T;
-    }
-    CK(cudaGetLastError());
+  int s0 = 0, from = 0;
+  for (int T : tb_schedule(b, nsteps)) {
+    const auto& w = b->tb_items.at(T);
+    launch_window_batch(b->mode, b->d_win, w.first, w.second, T, s0, from, s);
+    s0 += T;
+    from = 1 - from;
   }
+  CK(cudaGetLastError());
   if (!b->persistent || b->tb > 0) {
     void* fe = batch_phase_ptr(b->mode, b->maxp, b->rows, 0);
     void* fh = batch_phase_ptr(b->mode, b->maxp, b->rows, 1);
@@ -2470,8 +2693,7 @@ int fdtd_batch_tune(fdtd_batch* b, int steps) try {
     for (size_t q = 0; q < b->grids.size(); q++)
       if (b->cls[q] == c) b->mult[q] = keep;
   }
-  // temporal blocking with 2, 3 and 4 steps per launch, timed over whole
-  // pairs of launches
+  // temporal blocking of depths 2, 3 and 4, timed over whole pairs of launches
   float best_step = best / steps;
   int best_tb = 0;
   b->tb_ms.assign(3, 0.f);
@@ -2479,10 +2701,10 @@ int fdtd_batch_tune(fdtd_batch* b, int steps) try {
     rc = tb_prepare(b);
     if (!rc) rc = batch_items(b, best_rows);
     for (int depth = 2; depth <= 4 && !rc; depth++) {
-      const int n = (steps + 2 * depth - 1) / (2 * depth) * (2 * depth);
-      rc = tb_items(b, depth);
+      const int n = (steps + 4 * depth - 1) / (4 * depth) * (4 * depth);
       b->tb = depth;
-      if (!rc) rc = batch_launch(b, 2 * depth, b->stream);  // warm-up
+      rc = tb_ready(b, n);
+      if (!rc) rc = batch_launch(b, n, b->stream);  // warm-up
       if (!rc) rc = copy(false);
       CK(cudaEventRecord(e0, b->stream));
       if (!rc) rc = batch_launch(b, n, b->stream);
@@ -2498,7 +2720,6 @@ int fdtd_batch_tune(fdtd_batch* b, int steps) try {
       }
     }
     b->tb = 0;
-    if (!rc && best_tb) rc = tb_items(b, best_tb);
   }
   CK(cudaStreamSynchronize(b->stream));
   if (!best_tb) tb_release(b);  // the second copy is kept only while in use
@@ -2528,8 +2749,7 @@ int fdtd_batch_set_temporal(fdtd_batch* b, int depth) try {
   CK(cudaStreamSynchronize(b->stream));
   if (depth > 0) {
     if (const char* why = tb_unsupported(b)) return fail(FDTD_ERR_UNSUPPORTED, why);
-    int rc = tb_prepare(b);
-    if (!rc) rc = tb_items(b, depth);
+    const int rc = tb_prepare(b);
     if (rc) return rc;
   }
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
@@ -2615,6 +2835,8 @@ int fdtd_batch_step(fdtd_batch* b, int nsteps, void* stream) try {
   // from a CUDA graph
   auto it = b->graphs.find(nsteps);
   if (it == b->graphs.end()) {
+    const int trc = tb_ready(b, nsteps);
+    if (trc) return trc;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     int rc = batch_launch(b, nsteps, s);
     if (!rc) launch_batch_advance(b->d_ctrls, static_cast<int>(b->grids.size()), nsteps, s);
@@ -2629,10 +2851,11 @@ int fdtd_batch_step(fdtd_batch* b, int nsteps, void* stream) try {
     it = b->graphs.emplace(nsteps, exec).first;
   }
   CK(cudaGraphLaunch(it->second, s));
-  const long long tb_steps = b->tb > 0 ? nsteps / (2 * b->tb) * 2LL * b->tb : 0;
+  const long long windows = static_cast<long long>(tb_schedule(b, nsteps).size());
   for (auto* g : b->grids) {
     g->t += nsteps;
-    if (b->tb > 0) g->launches += tb_steps / b->tb + 2LL * (nsteps - tb_steps) + 1;
+    if (windows > 0) g->launches += windows + 1;
+    else if (b->tb > 0) g->launches += 2LL * nsteps + 1;
     else g->launches += b->persistent ? 2 : 2LL * nsteps + 1;
   }
   // later work on any member grid's own stream follows the batch

@@ -31,6 +31,32 @@ inline void once_per_device(const void* key, F set) {
   if (done.insert({dev, key}).second) set();
 }
 
+// Launches that follow one another on a stream (programmatic dependent
+// launch): a kernel launched with launch_chained may start once every CTA of
+// the one before it has called let_next_launch_start(); it reads nothing that
+// an earlier launch writes, and writes nothing, before after_previous_launch(),
+// which returns once the launch before has ended. Every kernel so launched
+// calls after_previous_launch() in each CTA, so a launch's end implies that of
+// all before it. Behind or before other launches both calls do nothing more
+// than stream order does.
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+
 // include/FDTDConstants.hpp:394-398
 constexpr double kPi = 3.14159265358979323846264338327950288;
 constexpr double kEps0 = 8.854e-12;
@@ -241,6 +267,61 @@ struct DftRegionDev {
   double* acc;  // [nf][npts][2]
 };
 
+// Temporal blocking of 2D FP32 grids (kernels_window.cu): windows of
+// kWinCols x 64 (or 32) cells take up to kWinMaxSteps steps per launch
+constexpr int kWinCols = 64, kWinRows = 64, kWinMaxSteps = 16;
+constexpr int kWinMaxBoxes = 8, kWinMaxRegions = 32;
+
+struct WinBox {  // box source, E (target 0) or H (2)
+  int comp, target, lo[2], hi[2], nvals;
+  const double* vals;
+};
+
+struct alignas(16) WinArgs {
+  int nx, ny, pitch;
+  int pml[2];
+  Slab slab[2];
+  // per axis: the cells lo..hi that are interior, outside the CPML slabs and
+  // have the plain (ungraded) profile values
+  int plain[2][2];
+  // the two copies of the state: TE Ex, Ey, Hz, TM Ez, Hx, Hy; the CPML
+  // integrators y and x of the E half, y and x of the H half; src_last
+  float* f[2][3];
+  float* psi[2][4];
+  double* src_last[2];
+  const float* ie;  // 1/eps per cell, or null: ie0 everywhere
+  float ie0;
+  float src_scale_d, src_scale_b, src_scale_h;
+  double eta;
+  Prof<float> prof[2][2];
+  int nsrc, nbox;
+  SourceDev src[kMaxSources];
+  WinBox box[kWinMaxBoxes];
+  int nreg[2];
+  const DftRegionDev* reg[2];
+  float* dft_buf[2];
+  long long dft_pts[2];
+  const Control* ctrl;
+  // adjoint forward (TM): the curl term d_t of every design cell after each
+  // step t, [step][row][column] over the design box dlo..dhi; null otherwise
+  float* cap;
+  int dlo[2], dhi[2];
+};
+
+// windows along an axis of n cells, each w cells wide, o of them its own
+// (the first and the last own their cells up to the axis' end)
+__host__ __device__ inline int window_tiles(int n, int w, int o) { return n <= w ? 1 : 1 + (n - w + o - 1) / o; }
+// windows of `rows` rows of an nx x ny grid taking T steps
+inline int window_count(int nx, int ny, int rows, int T) {
+  return window_tiles(nx, kWinCols, kWinCols - 2 * ((T + 1) & ~1)) * window_tiles(ny, rows, rows - 2 * T);
+}
+// T steps from copy `from` of the state to the other, s steps past the
+// counter; DFT samples go to ring slots slot .. slot + T - 1
+int launch_window(int mode, const WinArgs& a, int rows, int T, int s, int from, int slot, cudaStream_t st);
+// the same for the windows `items` ((grid << 24) | tile) of a batch
+int launch_window_batch(int mode, const WinArgs* grids, const unsigned* items, int nitems, int T, int s, int from,
+                        cudaStream_t st);
+
 // adjoint of the FP32 fused 2D TM step (kernels_adjoint.cu); all arrays in
 // the grid's pitch layout unless noted
 struct AdjArgs {
@@ -259,6 +340,24 @@ struct AdjArgs {
   int ndesign;
   double* grad;                     // dJ/deps_r, design box order
   const Control* ctrl;              // the grid's step counter
+};
+
+// The reversed steps in windows: what AdjArgs holds, on two copies of the
+// adjoint state
+struct AdjWinArgs {
+  int nx, ny, pitch;
+  int pml[2];
+  Slab slab[2];
+  int plain[2][2];     // as in WinArgs
+  float* f[2][3];      // adjoints of Ez, Hx, Hy
+  float* psi[2][4];    // of the integrators: xy (y slab), yx (x slab) of H; zx (x slab), zy (y slab) of E
+  const float* ie;
+  Prof<float> prof[2][2];
+  int plo[2], phi[2];
+  const float* force;  // [step][probe cell]: dJ/dEz of the probes after step t's E half
+  int dlo[2], dhi[2];
+  const float* store;  // [step][design cell]: d_t
+  double* grad;
 };
 
 // kernel launchers (stream-ordered); each returns the number of launches
@@ -315,6 +414,8 @@ int launch_dft_rebase(Control* ctrl, int nsamp, cudaStream_t s);
 int launch_dft_set_base(Control* ctrl, long long base, cudaStream_t s);
 int launch_finite_check(const void* p, long long n, int is_f32, int* flag, cudaStream_t s);
 int launch_step_advance(Control* ctrl, cudaStream_t s);
+// advances the step counter by n
+int launch_steps_advance(Control* ctrl, int n, cudaStream_t s);
 // advances the step counter and, if non-null, the one-launch step's epoch
 int launch_step_advance(Control* ctrl, unsigned* epoch, cudaStream_t s);
 // out[0] += sum over rows of (a*sa - b*sb)^2, out[1] += sum (b*sb)^2 (FP64)
@@ -337,7 +438,12 @@ struct BcFaces {
 };
 int launch_boundaries(const BcFaces& f, int ft, int is_f32, void* const* fields, int nx, int ny, int nz, int rowlen,
                       cudaStream_t s);
+// 1/eps of every cell of a 2D grid
 int launch_adjoint_inv_eps(const FusedArgs& fa, float* ie, cudaStream_t s);
+// force[t][p] = 2 Re(X_p e^{2 pi i f (t + 1)}) for t < nsteps
+int launch_adjoint_force(const double* X, double freq, int nprobe, int nsteps, float* force, cudaStream_t s);
+// reverses steps t, t - 1, .., t - T + 1 from copy `from` of the adjoint state to the other
+int launch_adjoint_window(const AdjWinArgs& a, int rows, int T, int t, int from, cudaStream_t s);
 int launch_adjoint_capture(const AdjArgs& a, const float* hx, const float* hy, float* slot, cudaStream_t s);
 int launch_adjoint_step(const AdjArgs& a, int back, const float* dslot, cudaStream_t s);
 int launch_box_source(int is_f32, void* field, const int* lo, const int* hi, int pitch, int ny, const double* vals,
@@ -352,13 +458,5 @@ struct BatchCtl {
 void* batch_kernel_ptr(int mode, int maxp, int rows);
 void* batch_phase_ptr(int mode, int maxp, int rows, int phase);
 int launch_batch_advance(Control* const* ctrls, int n, int nsteps, cudaStream_t s);
-// temporal blocking of a batch (depth 2, 3 or 4 steps per launch): the exact
-// tile of a window (*tw x *th cells; 0 for an unsupported depth), and one
-// launch over the tiles `items` that reads the state through `rd` and writes
-// it through `wr` (one FusedArgs per grid each), steps s .. s + depth - 1
-// past the counters
-int batch_tb_tile(int depth, int* tw, int* th);
-int launch_batch_tb(int mode, int depth, const FusedArgs* rd, const FusedArgs* wr, const unsigned* items,
-                    int nitems, int s, cudaStream_t st);
 
 }  // namespace fdtdb

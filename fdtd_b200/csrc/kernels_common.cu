@@ -335,6 +335,8 @@ __global__ void step_advance_kernel(Control* ctrl, unsigned* epoch) {
   if (epoch) *epoch += 1u;
 }
 
+__global__ void steps_advance_kernel(Control* ctrl, int n) { ctrl->t += n; }
+
 __global__ void chunk_start_kernel(Control* ctrl) { ctrl->t0 = ctrl->t; }
 __global__ void set_step_kernel(Control* ctrl, long long t) {
   ctrl->t = t;
@@ -466,6 +468,11 @@ int launch_batch_advance(Control* const* ctrls, int n, int nsteps, cudaStream_t 
 }
 
 int launch_step_advance(Control* ctrl, cudaStream_t s) { return launch_step_advance(ctrl, nullptr, s); }
+
+int launch_steps_advance(Control* ctrl, int n, cudaStream_t s) {
+  steps_advance_kernel<<<1, 1, 0, s>>>(ctrl, n);
+  return 1;
+}
 
 int launch_step_advance(Control* ctrl, unsigned* epoch, cudaStream_t s) {
   step_advance_kernel<<<1, 1, 0, s>>>(ctrl, epoch);

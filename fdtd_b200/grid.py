@@ -481,8 +481,9 @@ class Batch:
         _check(load_library().fdtd_batch_set_item_rows(self.h, _ip(rows_per_grid)))
 
     def set_temporal(self, depth: int) -> None:
-        """Temporal blocking: `depth` (2, 3 or 4) steps per launch from shared
-        memory, or 0 for off (fdtd_batch_set_temporal)."""
+        """Temporal blocking of depth 2, 3 or 4 (up to 2 * depth steps per
+        launch, in windows held on chip), or 0 for off
+        (fdtd_batch_set_temporal)."""
         _check(load_library().fdtd_batch_set_temporal(self.h, int(depth)))
 
     def temporal(self) -> dict:

@@ -214,6 +214,13 @@ int fdtd_dft_read(fdtd_grid* g, int handle, double* out);
 /* Advance nsteps full time steps on `stream` (a cudaStream_t, or NULL for the
  * handle's stream). Returns once the work is enqueued. */
 int fdtd_step(fdtd_grid* g, int nsteps, void* stream);
+/* 2D FP32 grids of non-dispersive materials with mu_r = 1, without TFSF
+ * planes, boundary conditions or DFT of surface quantities take calls of two
+ * steps or more in windows: several steps per launch, from one copy of the
+ * state into another (the grid holds a second copy of its fields and CPML
+ * integrators, and 1/eps per cell). Results are those of one launch per half
+ * step, which fdtd_set_sweep_kernel(g, FDTD_SWEEP_REGS) brings back, and
+ * which a grid keeps whose second copy finds no device memory. */
 /* Half a time step: phase 0 = the E half (curl of H, CPML, materials,
  * sources, TFSF, E-phase DFT sample; it also advances the TFSF aux grids one
  * step), phase 1 = the H half, which completes the step. The halves must
@@ -355,7 +362,7 @@ int fdtd_batch_destroy(fdtd_batch* b);
  * of 128 cells) for `steps` steps on a snapshot of the grids' state; then,
  * for the fastest, each size class of grids (quartiles of the cell counts,
  * largest first) in turn with work items 1, 2, 4 or 8 times that height;
- * then temporal blocking with 2, 3 and 4 steps per launch where the grids
+ * then temporal blocking of depths 2, 3 and 4 where the grids
  * allow it (which lays out the second copy of the state that mode needs);
  * restores the state and keeps the fastest. */
 int fdtd_batch_tune(fdtd_batch* b, int steps);
@@ -371,12 +378,13 @@ int fdtd_batch_item_rows(fdtd_batch* b, int* rows_per_grid, int* size_class, flo
 /* Set the work-item rows of every grid (in creation order): the tile height
  * in use times 1, 2, 4 or 8. The tuner's choice, by hand. */
 int fdtd_batch_set_item_rows(fdtd_batch* b, const int* rows_per_grid);
-/* Temporal blocking: each launch advances every grid `depth` steps (2, 3 or
- * 4) from shared memory, reading one copy of the state and writing a second
- * one that the batch allocates (the grids' fields, CPML integrators and
- * source values, once more); launches come in pairs, so the state ends in the
- * grids' own arrays, and the steps of a call beyond whole pairs run one kernel
- * per half step. Results equal the other launch modes bit for bit. Grids
+/* Temporal blocking of depth `depth` (2, 3 or 4): each launch advances every
+ * grid up to 2 * depth steps in windows held on chip, reading one copy of the
+ * state and writing a second one that the batch allocates (the grids' fields,
+ * CPML integrators and source values, once more, and 1/eps per cell); the
+ * launches of a call are even in number, so the state ends in the grids' own
+ * arrays, and a call of one step runs one kernel per half step. Results equal
+ * the other launch modes bit for bit. Grids
  * without dispersive materials whose sources lie inside their interiors
  * (FDTD_ERR_UNSUPPORTED otherwise); 0 turns it off. fdtd_batch_configure turns
  * it off too; fdtd_batch_tune also times depths 2, 3 and 4 and keeps one if
