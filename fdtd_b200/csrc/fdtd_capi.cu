@@ -1513,8 +1513,10 @@ int fdtd_dft_read(fdtd_grid* g, int handle, double* out) try {
 }
 
 static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof);
+static void adjoint_capture_args(fdtd_adjoint* a, WinArgs& w);
+static int adjoint_capture_step(fdtd_adjoint* a, long long t, cudaStream_t s);
 static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof);
-static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s);
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoint* adj = nullptr);
 
 // The TFSF aux tables for a call of nsteps steps: at least 257 rows, so that
 // calls of up to 256 steps keep them (and the step graph, whose launches hold
@@ -1726,13 +1728,17 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
 // of launches per stretch of steps (ending on the grid's own arrays), each
 // stretch within the DFT sample ring; a single step left over goes out as
 // launches per half step.
-static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s) {
+// `adj`: the curl terms of the design cells of every step go to its store.
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoint* adj) {
+  WinArgs wa = g->win;
+  if (adj) adjoint_capture_args(adj, wa);
   const bool dft = !g->dfts.empty();
   int rows = kWinRows;
   const int T = window_steps(g->n[0], g->n[1], &rows);
   for (int done = 0; done < nsteps;) {
     const int n = std::min(nsteps - done, kDftChunk - (dft ? g->dft_pending : 0));
     if (n == 1) {
+      if (adj) g->launches += adjoint_capture_step(adj, done, s);
       const int rc = enqueue_steps(g, 1, s, nullptr);
       if (rc) return rc;
       done++;
@@ -1742,7 +1748,7 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s) {
     for (int q = 0; q < L; q++) {
       const int at = static_cast<int>(static_cast<long long>(n) * q / L);
       const int t = static_cast<int>(static_cast<long long>(n) * (q + 1) / L) - at;
-      g->launches += launch_window(g->d.mode, g->win, rows, t, at, q & 1, g->dft_pending + at, s);
+      g->launches += launch_window(g->d.mode, wa, rows, t, at, q & 1, g->dft_pending + at, s);
     }
     g->launches += launch_steps_advance(g->ctrl, n, s);
     if (dft) {
@@ -3075,6 +3081,11 @@ struct fdtd_adjoint {
   float* d_store = nullptr;
   double* d_X = nullptr;
   double* d_grad = nullptr;
+  // d_t of every design cell and step, kept by the forward (no checkpoints
+  // and no recomputation then), and the adjoint state's two copies
+  float* d_dt = nullptr;
+  float* d_force = nullptr;
+  float* win[2][7] = {};  // aez, ahx, ahy, then the integrators xy, yx, zx, zy
   double J = 0.0;
   std::map<int, cudaGraphExec_t> graphs;  // one replayable segment per length
   std::map<int, long long> graph_launches;
@@ -3101,6 +3112,115 @@ static int adj_copy_state(fdtd_adjoint* a, char* base, bool save, cudaStream_t s
     CK(cudaMemcpyAsync(save ? sp : st.first, save ? st.first : sp, st.second, cudaMemcpyDeviceToDevice, s));
     off += (st.second + 255) / 256 * 256;
   }
+  return FDTD_OK;
+}
+
+static int adj_design(const fdtd_adjoint* a) {
+  return (a->dhi[0] - a->dlo[0] + 1) * (a->dhi[1] - a->dlo[1] + 1);
+}
+
+static void adjoint_capture_args(fdtd_adjoint* a, WinArgs& w) {
+  w.cap = a->d_dt;
+  for (int d = 0; d < 2; d++) {
+    w.dlo[d] = a->dlo[d];
+    w.dhi[d] = a->dhi[d];
+  }
+}
+
+// d_t of step t ahead of that step
+static int adjoint_capture_step(fdtd_adjoint* a, long long t, cudaStream_t s) {
+  const FusedArgs fa = fused_args(a->g);
+  AdjArgs aa;
+  memset(&aa, 0, sizeof(aa));
+  aa.pitch = fa.pitch;
+  for (int x = 0; x < 3; x++) aa.prof[0][x] = fa.prof[0][x];
+  for (int d = 0; d < 2; d++) {
+    aa.dlo[d] = a->dlo[d];
+    aa.dhi[d] = a->dhi[d];
+  }
+  aa.ndesign = adj_design(a);
+  return launch_adjoint_capture(aa, fa.H[0], fa.H[1], a->d_dt + t * aa.ndesign, s);
+}
+
+// The forward of a grid that takes its steps in windows, keeping d_t of every
+// design cell: the backward then needs neither the forward's states nor its
+// steps again. *done says whether it ran: not for a grid that keeps the
+// launches per half step, nor where the terms would take more than a
+// sixteenth of the device's memory (checkpoints and recomputation then).
+static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
+  fdtd_grid* g = a->g;
+  *done = false;
+  int rc = ensure_pml(g);
+  if (!rc) rc = ensure_window(g);
+  if (rc || !g->win_ok) return rc;
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  const size_t bytes = static_cast<size_t>(nsteps) * adj_design(a) * sizeof(float);
+  const size_t np = static_cast<size_t>(a->phi[0] - a->plo[0] + 1) * (a->phi[1] - a->plo[1] + 1);
+  const size_t fbytes = static_cast<size_t>(nsteps) * np * sizeof(float);
+  if (bytes > total_b / 16 || fbytes > total_b / 16) return FDTD_OK;
+  rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_dt), bytes);
+  if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_force), fbytes);
+  if (rc) {
+    a->d_dt = nullptr;
+    return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
+  }
+  if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
+  rc = enqueue_windows(g, nsteps, g->stream, a);
+  if (rc) return rc;
+  g->t += nsteps;
+  *done = true;
+  return FDTD_OK;
+}
+
+// the backward from the stored terms: every step reversed in windows
+static int adj_backward_stored(fdtd_adjoint* a, const FusedArgs& fa) {
+  fdtd_grid* g = a->g;
+  cudaStream_t s = g->stream;
+  const size_t fe = static_cast<size_t>(field_elems(g));
+  const size_t sx = static_cast<size_t>(g->n[1]) * g->slab[0].W4, sy = static_cast<size_t>(g->slab[1].W) * rowlen(g);
+  const size_t elems[7] = {fe, fe, fe, sy, sx, sx, sy};
+  const int np = (a->phi[0] - a->plo[0] + 1) * (a->phi[1] - a->plo[1] + 1);
+  for (int c = 0; c < 2; c++)
+    for (int q = 0; q < 7; q++) {
+      if (!a->win[c][q]) {
+        const int rc = adj_alloc(a, reinterpret_cast<void**>(&a->win[c][q]), elems[q] * sizeof(float));
+        if (rc) return rc;
+      }
+      CK(cudaMemsetAsync(a->win[c][q], 0, std::max<size_t>(elems[q], 4) * sizeof(float), s));
+    }
+  AdjWinArgs w;
+  memset(&w, 0, sizeof(w));
+  const WinArgs& f = g->win;
+  w.nx = f.nx;
+  w.ny = f.ny;
+  w.pitch = f.pitch;
+  for (int x = 0; x < 2; x++) {
+    w.pml[x] = f.pml[x];
+    w.slab[x] = f.slab[x];
+    for (int q = 0; q < 2; q++) w.plain[x][q] = f.plain[x][q];
+    for (int h = 0; h < 2; h++) w.prof[h][x] = fa.prof[h][x];
+    w.plo[x] = a->plo[x];
+    w.phi[x] = a->phi[x];
+    w.dlo[x] = a->dlo[x];
+    w.dhi[x] = a->dhi[x];
+  }
+  for (int c = 0; c < 2; c++) {
+    for (int q = 0; q < 3; q++) w.f[c][q] = a->win[c][q];
+    for (int q = 0; q < 4; q++) w.psi[c][q] = a->win[c][3 + q];
+  }
+  w.ie = a->d_ie;
+  w.force = a->d_force;
+  w.store = a->d_dt;
+  w.grad = a->d_grad;
+  g->launches += launch_adjoint_force(a->d_X, a->freq, np, static_cast<int>(a->nsteps), a->d_force, s);
+  int rows = kWinRows, from = 0;
+  const int T = window_steps(g->n[0], g->n[1], &rows);
+  for (int t = static_cast<int>(a->nsteps) - 1; t >= 0; t -= T) {
+    g->launches += launch_adjoint_window(w, rows, std::min(T, t + 1), t, from, s);
+    from = 1 - from;
+  }
+  CK(cudaGetLastError());
   return FDTD_OK;
 }
 
@@ -3211,20 +3331,25 @@ int fdtd_adjoint_forward(fdtd_adjoint* a, int nsteps, double* J) try {
     if (rc) return rc;
   }
   cudaStream_t s = g->stream;
-  a->state = grid_state(g);
-  a->state_bytes = 0;
-  for (auto& st : a->state) a->state_bytes += (st.second + 255) / 256 * 256;
-  a->nckpt = (nsteps + a->ckpt_every - 1) / a->ckpt_every;
-  int rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_ckpt), a->state_bytes * a->nckpt);
-  if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_final), a->state_bytes);
+  bool stored = false;
+  int rc = adj_forward_stored(a, nsteps, &stored);
   if (rc) return rc;
-  for (int q = 0; q < a->nckpt; q++) {
-    rc = adj_copy_state(a, a->d_ckpt + a->state_bytes * q, true, s);
-    if (!rc) rc = step_impl(g, std::min(a->ckpt_every, nsteps - q * a->ckpt_every), nullptr, nullptr);
+  if (!stored) {
+    a->state = grid_state(g);
+    a->state_bytes = 0;
+    for (auto& st : a->state) a->state_bytes += (st.second + 255) / 256 * 256;
+    a->nckpt = (nsteps + a->ckpt_every - 1) / a->ckpt_every;
+    rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_ckpt), a->state_bytes * a->nckpt);
+    if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_final), a->state_bytes);
+    if (rc) return rc;
+    for (int q = 0; q < a->nckpt; q++) {
+      rc = adj_copy_state(a, a->d_ckpt + a->state_bytes * q, true, s);
+      if (!rc) rc = step_impl(g, std::min(a->ckpt_every, nsteps - q * a->ckpt_every), nullptr, nullptr);
+      if (rc) return rc;
+    }
+    rc = adj_copy_state(a, a->d_final, true, s);
     if (rc) return rc;
   }
-  rc = adj_copy_state(a, a->d_final, true, s);
-  if (rc) return rc;
   const DftH& r = g->dfts[a->dft];
   rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_X), static_cast<size_t>(r.npts) * 2 * sizeof(double));
   if (rc) return rc;
@@ -3255,6 +3380,20 @@ int fdtd_adjoint_backward(fdtd_adjoint* a, double* grad) try {
   int rc = FDTD_OK;
   if (!a->d_ie) {
     rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_ie), fe * sizeof(float));
+    if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_grad), nd * sizeof(double));
+    if (rc) return rc;
+  }
+  if (a->d_dt) {
+    const FusedArgs fa = fused_args(g);
+    g->launches += launch_adjoint_inv_eps(fa, a->d_ie, s);
+    CK(cudaMemsetAsync(a->d_grad, 0, nd * sizeof(double), s));
+    rc = adj_backward_stored(a, fa);
+    if (rc) return rc;
+    CK(cudaMemcpyAsync(grad, a->d_grad, nd * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return FDTD_OK;
+  }
+  if (!a->d_store) {
     for (int q = 0; q < 7 && !rc; q++) rc = adj_alloc(a, reinterpret_cast<void**>(&a->adj[q]), fe * sizeof(float));
     // adjoint CPML integrators: the compact slabs of psi_zx, psi_zy (E) and psi_yx, psi_xy (H)
     const size_t sx = static_cast<size_t>(g->n[1]) * g->slab[0].W, sy = static_cast<size_t>(g->slab[1].W) * rowlen(g);
@@ -3264,7 +3403,6 @@ int fdtd_adjoint_backward(fdtd_adjoint* a, double* grad) try {
       rc = adj_alloc(a, reinterpret_cast<void**>(&a->apsi[q]), sizes[q] * sizeof(float));
     }
     if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_store), static_cast<size_t>(a->ckpt_every) * nd * sizeof(float));
-    if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_grad), nd * sizeof(double));
     if (rc) return rc;
   }
   FusedArgs fa = fused_args(g);

@@ -410,8 +410,11 @@ int fdtd_batch_error_flags(fdtd_batch* b, int* flags);
  * fdtd_add_dft). The grid must be unstepped, without TFSF planes or
  * dispersive materials; the design box must lie outside the CPML and hold no
  * D-target source. create adds the probe DFT region to the grid. forward
- * steps the grid nsteps times, checkpointing the state every ckpt_every
- * steps, and returns J; backward recomputes each segment from its checkpoint,
+ * steps the grid nsteps times and returns J, keeping one FP32 value per
+ * design cell and step where these take at most a sixteenth of the device's
+ * memory (and the grid takes its steps in windows, see fdtd_step), else
+ * checkpointing the state every ckpt_every steps; backward reverses the steps
+ * from the kept values, or recomputes each segment from its checkpoint and
  * reverses it, leaves the grid in its post-forward state and writes
  * dJ/deps_r of every design cell (x fastest) to the host array grad. One
  * forward and one backward per handle; destroy it before its grid.
