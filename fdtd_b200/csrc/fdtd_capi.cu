@@ -1255,14 +1255,14 @@ int fdtd_add_source_box(fdtd_grid* g, int comp, int target, const int* lo, const
 
 // the box sources of one phase (0 = E, 1 = H): shift 0 adds this step's
 // value, shift -1 takes back the previous step's (fused method only)
-static int launch_boxes(fdtd_grid* g, int phase, int shift, cudaStream_t s) {
+static int launch_boxes(fdtd_grid* g, int phase, int shift, cudaStream_t s, int ts = 0) {
   int n = 0;
   for (const auto& b : g->boxes) {
     if ((b.target == 0) != (phase == 0)) continue;
     void* f = phase == 0 ? g->E[b.comp] : g->H[b.comp];
     const double scale = (phase == 1 && g->f32 ? eta() : 1.0) * (shift < 0 ? -1.0 : 1.0);
     n += launch_box_source(g->f32 ? 1 : 0, f, b.lo, b.hi, static_cast<int>(rowlen(g)), g->n[1], b.d_vals, b.nvals,
-                           scale, shift, g->ctrl, s);
+                           scale, shift + ts, g->ctrl, s);
   }
   return n;
 }
@@ -1641,7 +1641,13 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
     eh.epoch = g->d_eh;
     eh.flags = g->d_eh + 1;
   }
+  // the kernels take the step as counter + offset, so that the counter moves
+  // once per call (per step where the one-launch step's epoch follows it, or
+  // its time is measured)
+  const bool each = use_eh || prof;
   for (int q = 0; q < nsteps; q++) {
+    const int ts = each ? 0 : q;
+    fa.ts = pa.ts = ts;
     if (prof) CK(cudaEventRecord(ev[0], s));
     if (use_eh) {
       g->launches += launch_staged_eh(fa, eh, eh_blocks, s);
@@ -1668,7 +1674,7 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
       }
       continue;
     }
-    if (boxes && g->f32) g->launches += launch_boxes(g, 0, -1, s);
+    if (boxes && g->f32) g->launches += launch_boxes(g, 0, -1, s, ts);
     if (g->f32) {
       g->launches += use_tma      ? launch_tma_e(fa, g->tma, s)
                      : use_staged ? launch_staged_e(fa, s)
@@ -1682,12 +1688,12 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
     }
     if (prof) CK(cudaEventRecord(ev[1], s));
     if (g->f32) g->launches += launch_tfsf_fused(mode, fa, 0, s);
-    if (boxes) g->launches += launch_boxes(g, 0, 0, s);
+    if (boxes) g->launches += launch_boxes(g, 0, 0, s, ts);
     g->launches += launch_bc(g, 0, s);
     g->launches += launch_dft_gather(g->f32 ? 1 : 0, g->d_dft[0], g->ndft[0], g->dft_pts[0], g->dft_maxpts[0], fE, g->n[1],
                                      static_cast<int>(rowlen(g)), g->dft_pending, g->d_dft_buf[0], s);
     if (prof) CK(cudaEventRecord(ev[2], s));
-    if (boxes && g->f32) g->launches += launch_boxes(g, 1, -1, s);
+    if (boxes && g->f32) g->launches += launch_boxes(g, 1, -1, s, ts);
     if (g->f32) {
       g->launches += use_tma      ? launch_tma_h(fa, g->tma, s)
                      : use_staged ? launch_staged_h(fa, s)
@@ -1701,12 +1707,12 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
     }
     if (prof) CK(cudaEventRecord(ev[3], s));
     if (g->f32) g->launches += launch_tfsf_fused(mode, fa, 1, s);
-    if (boxes) g->launches += launch_boxes(g, 1, 0, s);
+    if (boxes) g->launches += launch_boxes(g, 1, 0, s, ts);
     g->launches += launch_bc(g, 1, s);
     g->launches += launch_dft_gather(g->f32 ? 1 : 0, g->d_dft[1], g->ndft[1], g->dft_pts[1], g->dft_maxpts[1], fH, g->n[1],
                                      static_cast<int>(rowlen(g)), g->dft_pending, g->d_dft_buf[1], s);
     if (prof) CK(cudaEventRecord(ev[4], s));
-    g->launches += launch_step_advance(g->ctrl, s);
+    if (each) g->launches += launch_step_advance(g->ctrl, s);
     if (!g->dfts.empty() && ++g->dft_pending == kDftChunk) g->launches += flush_dft(g, s);
     if (prof) {
       CK(cudaEventRecord(ev[5], s));
@@ -1718,6 +1724,7 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
       }
     }
   }
+  if (!each) g->launches += launch_steps_advance(g->ctrl, nsteps, s);
   if (prof)
     for (auto& e : ev) cudaEventDestroy(e);
   if (g->dft_pending > 0) g->launches += flush_dft(g, s);

@@ -105,7 +105,7 @@ __device__ __forceinline__ GroupCtx make_ctx(const FusedArgs& a, int ft, int x4,
   g.uniform_mat = !a.ids && !a.bids;
   g.fsx = ld4(a.prof[ft][0].F + x4);
   g.fsy = a.prof[ft][1].F[min(j, a.ny - 2)];
-  g.t = a.ctrl->t;
+  g.t = a.ctrl->t;  // of the counter; a.ts is added where a source reads it
   return g;
 }
 
@@ -198,7 +198,8 @@ __device__ __forceinline__ void e_group_update(const FusedArgs& a, const GroupCt
       const SourceDev& sr = a.src[q];
       if (sr.target > 1 || sr.j != j || sr.k != k || sr.i < x4 || sr.i >= x4 + 4) continue;
       const int e = sr.i - x4;
-      const double v = g.t < sr.nvals ? sr.vals[g.t] : 0.0;
+      const long long t = g.t + a.ts;
+      const double v = t < sr.nvals ? sr.vals[t] : 0.0;
       if (sr.target == 1) {
         const float dv = static_cast<float>(v * a.src_scale_d);
         if (sr.comp == 0) set_el(dX, e, el(dX, e) + dv);
@@ -377,7 +378,8 @@ __device__ __forceinline__ void h_group_update(const FusedArgs& a, const GroupCt
       const SourceDev& sr = a.src[q];
       if (sr.target < 2 || sr.j != j || sr.k != k || sr.i < x4 || sr.i >= x4 + 4) continue;
       const int e = sr.i - x4;
-      const double v = g.t < sr.nvals ? sr.vals[g.t] : 0.0;
+      const long long t = g.t + a.ts;
+      const double v = t < sr.nvals ? sr.vals[t] : 0.0;
       if (sr.target == 3) {
         const float dv = static_cast<float>(v * a.src_scale_b);
         if (sr.comp == 0) set_el(dX, e, el(dX, e) - dv);

@@ -42,6 +42,11 @@ inline void once_per_device(const void* key, F set) {
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void after_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+constexpr unsigned long long kChainCtas = 16384;
+// whether a launch of this many CTAs is chained: one of many rounds of CTAs
+// gains nothing worth their waits
+inline bool chains(dim3 grid) { return static_cast<unsigned long long>(grid.x) * grid.y * grid.z <= kChainCtas; }
+
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -53,7 +58,7 @@ inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chains(grid) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, fn, P(args)...);
 }
 
@@ -204,6 +209,7 @@ struct PlainArgs {
   PlaneDev planes[kMaxPlanes];
   AuxTab aux[kMaxPlanes];
   Control* ctrl;
+  int ts;  // this step's number past the counter
   // time policy of the curl updates (include/YeeUpdates.hpp:182-294): bd
   // history levels (0 BD1, 2 BD3, 3 BD4), bdk the coefficients of
   // TimePolicy::get, cc its curl_coeff; hist[D|B][level][comp]
@@ -249,6 +255,7 @@ struct FusedArgs {
   double dx, dt;
   double eta;
   Control* ctrl;
+  int ts;  // this step's number past the counter
   int item_rows;  // batches: rows of one work item of this grid (a multiple of the kernel's rows; 0: the kernel's)
   int kbeg, kend;  // the staged 3D sweeps update planes kbeg .. kend-1 (all interior planes: 1 .. nz-2)
 };

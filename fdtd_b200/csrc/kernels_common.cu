@@ -76,6 +76,8 @@ template <typename R>
 __global__ void __launch_bounds__(256) dft_gather_kernel(const DftRegionDev* __restrict__ regions, long long total,
                                                          const R* const* __restrict__ fields, int ny, int pitch,
                                                          long long slot, R* buf) {
+  after_previous_launch();
+  let_next_launch_start();
   const DftRegionDev& g = regions[blockIdx.y];
   const int q0 = blockIdx.x * (256 * kGatherPts) + threadIdx.x;
   if (q0 >= g.npts) return;
@@ -217,11 +219,13 @@ int launch_dft_gather(int precision, const DftRegionDev* regions, int nreg, long
   if (nreg == 0 || total_pts == 0) return 0;
   const dim3 grid(static_cast<unsigned>((max_pts + 256 * kGatherPts - 1) / (256 * kGatherPts)), nreg);
   if (precision == 0)
-    dft_gather_kernel<double><<<grid, 256, 0, s>>>(regions, total_pts, reinterpret_cast<const double* const*>(fields),
-                                                   ny, pitch, slot, static_cast<double*>(buf));
+    launch_chained(dft_gather_kernel<double>, grid, dim3(256), 0, s, regions, total_pts,
+                   reinterpret_cast<const double* const*>(fields), ny, pitch, static_cast<long long>(slot),
+                   static_cast<double*>(buf));
   else
-    dft_gather_kernel<float><<<grid, 256, 0, s>>>(regions, total_pts, reinterpret_cast<const float* const*>(fields),
-                                                  ny, pitch, slot, static_cast<float*>(buf));
+    launch_chained(dft_gather_kernel<float>, grid, dim3(256), 0, s, regions, total_pts,
+                   reinterpret_cast<const float* const*>(fields), ny, pitch, static_cast<long long>(slot),
+                   static_cast<float*>(buf));
   return 1;
 }
 
@@ -364,6 +368,8 @@ __host__ __device__ float bc_sign(int kind, int ft, int c, int axis) {
 template <typename T>
 __global__ void __launch_bounds__(256) boundary_kernel(BcFaces f, int ft, T* f0, T* f1, T* f2, int nx, int ny,
                                                        int nz, int rowlen) {
+  after_previous_launch();
+  let_next_launch_start();
   const BcFace& b = f.face[blockIdx.z];
   const int ua = b.axis == 0 ? 1 : 0, va = b.axis == 2 ? 1 : 2;  // transverse axes
   const int n[3] = {nx, ny, nz};
@@ -403,12 +409,11 @@ int launch_boundaries(const BcFaces& f, int ft, int is_f32, void* const* fields,
   const dim3 block(32, 8, 1);
   const dim3 grid(static_cast<unsigned>((mu + 31) / 32), static_cast<unsigned>((mv + 7) / 8), f.n);
   if (is_f32)
-    boundary_kernel<float><<<grid, block, 0, s>>>(f, ft, static_cast<float*>(fields[0]), static_cast<float*>(fields[1]),
-                                                  static_cast<float*>(fields[2]), nx, ny, nz, rowlen);
+    launch_chained(boundary_kernel<float>, grid, block, 0, s, f, ft, static_cast<float*>(fields[0]),
+                   static_cast<float*>(fields[1]), static_cast<float*>(fields[2]), nx, ny, nz, rowlen);
   else
-    boundary_kernel<double><<<grid, block, 0, s>>>(f, ft, static_cast<double*>(fields[0]),
-                                                   static_cast<double*>(fields[1]), static_cast<double*>(fields[2]),
-                                                   nx, ny, nz, rowlen);
+    launch_chained(boundary_kernel<double>, grid, block, 0, s, f, ft, static_cast<double*>(fields[0]),
+                   static_cast<double*>(fields[1]), static_cast<double*>(fields[2]), nx, ny, nz, rowlen);
   return 1;
 }
 
@@ -429,6 +434,8 @@ int launch_set_step(Control* ctrl, long long t, cudaStream_t s) {
 template <typename T>
 __global__ void box_source_kernel(T* f, int lox, int loy, int loz, int ex, int ey, long long n, int pitch, int ny,
                                   const double* vals, int nvals, double scale, int shift, const Control* ctrl) {
+  after_previous_launch();
+  let_next_launch_start();
   const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long t = ctrl->t + shift;
   if (q >= n || t < 0 || t >= nvals) return;
@@ -446,11 +453,11 @@ int launch_box_source(int is_f32, void* field, const int* lo, const int* hi, int
   const long long n = static_cast<long long>(ex) * ey * ez;
   const unsigned blocks = static_cast<unsigned>((n + 255) / 256);
   if (is_f32)
-    box_source_kernel<float><<<blocks, 256, 0, s>>>(static_cast<float*>(field), lo[0], lo[1], lo[2], ex, ey, n, pitch,
-                                                    ny, vals, nvals, scale, shift, ctrl);
+    launch_chained(box_source_kernel<float>, dim3(blocks), dim3(256), 0, s, static_cast<float*>(field), lo[0], lo[1],
+                   lo[2], ex, ey, n, pitch, ny, vals, nvals, scale, shift, ctrl);
   else
-    box_source_kernel<double><<<blocks, 256, 0, s>>>(static_cast<double*>(field), lo[0], lo[1], lo[2], ex, ey, n,
-                                                     pitch, ny, vals, nvals, scale, shift, ctrl);
+    launch_chained(box_source_kernel<double>, dim3(blocks), dim3(256), 0, s, static_cast<double*>(field), lo[0], lo[1],
+                   lo[2], ex, ey, n, pitch, ny, vals, nvals, scale, shift, ctrl);
   return 1;
 }
 

@@ -39,6 +39,8 @@ __device__ __forceinline__ bool range_hits_slab(const Slab& s, int lo, int hi) {
 
 template <int MODE, int MAXP>
 __global__ void __launch_bounds__(256) fused_e_kernel(const __grid_constant__ FusedArgs a, int kchunk) {
+  after_previous_launch();
+  let_next_launch_start();
   const int lane = threadIdx.x;
   const int i0 = blockIdx.x * 32 + 1, j0 = blockIdx.y * kBY + 1;
   const int i = i0 + lane, j = j0 + threadIdx.y;
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(256) fused_e_kernel(const __grid_constant__ Fu
     kend = min(kbeg + kchunk, a.nz - 1);
   }
   const long long sy = a.pitch, sz = static_cast<long long>(a.pitch) * a.ny;
-  const long long t = a.ctrl->t;
+  const long long t = a.ctrl->t + a.ts;
   // CTA-level feature tests
   const int i1 = min(i0 + 31, a.nx - 2), j1 = min(j0 + kBY - 1, a.ny - 2);
   bool pml_x = a.pml_axis[0] && range_hits_slab(a.slab[0], i0, i1);
@@ -181,6 +183,8 @@ __global__ void __launch_bounds__(256) fused_e_kernel(const __grid_constant__ Fu
 
 template <int MODE>
 __global__ void __launch_bounds__(256) fused_h_kernel(const __grid_constant__ FusedArgs a, int kchunk) {
+  after_previous_launch();
+  let_next_launch_start();
   const int lane = threadIdx.x;
   const int i0 = blockIdx.x * 32 + 1, j0 = blockIdx.y * kBY + 1;
   const int i = i0 + lane, j = j0 + threadIdx.y;
@@ -262,7 +266,7 @@ __global__ void __launch_bounds__(256) fused_h_kernel(const __grid_constant__ Fu
     for (int s = 0; s < a.nsrc; s++) {
       const SourceDev& sr = a.src[s];
       if (sr.target < 2 || sr.cell != c) continue;
-      const long long t = a.ctrl->t;
+      const long long t = a.ctrl->t + a.ts;
       const double v = t < sr.nvals ? sr.vals[t] : 0.0;
       if (sr.target == 3) {
         const float dv = static_cast<float>(v * a.src_scale_b);
@@ -310,7 +314,7 @@ static int launch_e_t(const FusedArgs& a, cudaStream_t s) {
     kchunk = kchunk_for(a.nz, bx * by);
     bz = (a.nz - 2 + kchunk - 1) / kchunk;
   }
-  fused_e_kernel<MODE, MAXP><<<dim3(bx, by, bz), block, 0, s>>>(a, kchunk);
+  launch_chained(fused_e_kernel<MODE, MAXP>, dim3(bx, by, bz), block, 0, s, a, kchunk);
   return 1;
 }
 
@@ -341,7 +345,7 @@ static int launch_h_t(const FusedArgs& a, cudaStream_t s) {
     kchunk = kchunk_for(a.nz, bx * by);
     bz = (a.nz - 2 + kchunk - 1) / kchunk;
   }
-  fused_h_kernel<MODE><<<dim3(bx, by, bz), block, 0, s>>>(a, kchunk);
+  launch_chained(fused_h_kernel<MODE>, dim3(bx, by, bz), block, 0, s, a, kchunk);
   return 1;
 }
 

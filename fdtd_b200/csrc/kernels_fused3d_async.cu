@@ -116,8 +116,15 @@ __device__ __forceinline__ void e_tile(const FusedArgs& a, int bx, int by, int k
                        PJ ? s + kSlotsE * kThreads : nullptr, kThreads);
 }
 
-template <int MAXP, int MINB, bool PJ>
+// CHAIN: launched behind a kernel that may still run (launch_chained); sweeps
+// of very many CTAs are launched without (the wait alone, taken by each of
+// 882k CTAs, cost the 768^3 step 1.5%)
+template <int MAXP, int MINB, bool PJ, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, MINB) staged_e_kernel(const __grid_constant__ FusedArgs a) {
+  if (CHAIN) {
+    after_previous_launch();
+    let_next_launch_start();
+  }
   extern __shared__ float4 sm[];
   e_tile<MAXP, PJ>(a, blockIdx.x, blockIdx.y, a.kbeg + blockIdx.z, sm);
 }
@@ -162,8 +169,12 @@ __device__ __forceinline__ void h_tile(const FusedArgs& a, int bx, int by, int k
                  ez_xp3, s[7 * kThreads], s[8 * kThreads], s[9 * kThreads], px);
 }
 
-template <int MINB, bool MU>
+template <int MINB, bool MU, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, MINB) staged_h_kernel(const __grid_constant__ FusedArgs a) {
+  if (CHAIN) {
+    after_previous_launch();
+    let_next_launch_start();
+  }
   extern __shared__ float4 sm[];
   // planes from the top down, as the flat H sweep
   h_tile<MU>(a, blockIdx.x, blockIdx.y, a.kend - 1 - blockIdx.z, sm);
@@ -182,21 +193,29 @@ static int carveout_for(int ctas, size_t smem) {
   return static_cast<int>(std::min<size_t>(100, (need * 100 + max_sm - 1) / max_sm));
 }
 
+static dim3 sweep_grid(const FusedArgs& a) {
+  const unsigned planes = a.kend - a.kbeg;
+  return dim3(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, planes);
+}
+
 // CTAs per SM: 7 (6 for two poles) with the ADE state read per component;
 // with it staged, as many as the shared memory holds (two poles: 4 x 49.7 KB)
 template <int MAXP, bool PJ>
 static void staged_e_launch(const FusedArgs& a, cudaStream_t s) {
-  dim3 grid(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, a.kend - a.kbeg), block(32, kRowsA, 1);
+  const dim3 block(32, kRowsA, 1);
   constexpr int slots = kSlotsE + (PJ ? pj_slots<MAXP>() : 0);
   constexpr int minb = !PJ ? (MAXP >= 2 ? 6 : 7) : (MAXP >= 2 ? 4 : (MAXP == 1 ? 6 : 7));
   const size_t smem = slots * kThreads * sizeof(float4) + kThreads * sizeof(unsigned);
-  auto fn = staged_e_kernel<MAXP, minb, PJ>;
-  // once per device: the shared-memory split that holds minb CTAs, the rest as L1
-  once_per_device(reinterpret_cast<const void*>(fn), [&] {
-    cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(minb, smem));
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  });
-  fn<<<grid, block, smem, s>>>(a);
+  auto go = [&](auto fn) {
+    // once per device: the shared-memory split that holds minb CTAs, the rest as L1
+    once_per_device(reinterpret_cast<const void*>(fn), [&] {
+      cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(minb, smem));
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    });
+    launch_chained(fn, sweep_grid(a), block, smem, s, a);
+  };
+  const bool chain = chains(sweep_grid(a));
+  chain ? go(staged_e_kernel<MAXP, minb, PJ, true>) : go(staged_e_kernel<MAXP, minb, PJ, false>);
 }
 
 template <int MAXP>
@@ -222,12 +241,16 @@ int launch_staged_e(const FusedArgs& a, cudaStream_t s) {
 
 template <bool MU>
 static void staged_h_dispatch(const FusedArgs& a, cudaStream_t s) {
-  dim3 grid(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, a.kend - a.kbeg), block(32, kRowsA, 1);
+  const dim3 block(32, kRowsA, 1);
   const size_t smem = kSlotsH * kThreads * sizeof(float4);
-  once_per_device(reinterpret_cast<const void*>(staged_h_kernel<8, MU>), [&] {
-    cudaFuncSetAttribute(staged_h_kernel<8, MU>, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(8, smem));
-  });
-  staged_h_kernel<8, MU><<<grid, block, smem, s>>>(a);
+  auto go = [&](auto fn) {
+    once_per_device(reinterpret_cast<const void*>(fn), [&] {
+      cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(8, smem));
+    });
+    launch_chained(fn, sweep_grid(a), block, smem, s, a);
+  };
+  const bool chain = chains(sweep_grid(a));
+  chain ? go(staged_h_kernel<8, MU, true>) : go(staged_h_kernel<8, MU, false>);
 }
 
 int launch_staged_h(const FusedArgs& a, cudaStream_t s) {

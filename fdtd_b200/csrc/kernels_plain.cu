@@ -13,6 +13,8 @@
 //
 // This file is compiled with -fmad=false: no multiply-add contraction, so each
 // product and sum rounds as in the reference compiled with -ffp-contract=off.
+#include <algorithm>
+
 #include "internal.h"
 
 namespace fdtdb {
@@ -81,6 +83,8 @@ __device__ __forceinline__ long long plane_cell(const PlaneDev& p, int i, int j,
 // in-plane axis, z over the planes.
 template <int MODE>
 __global__ void __launch_bounds__(128) tfsf_pre_kernel(const __grid_constant__ PlainArgs a, int ft) {
+  after_previous_launch();
+  let_next_launch_start();
   const PlaneDev& p = a.planes[blockIdx.z];
   const int u = p.axis == 0 ? 1 : 0, v = p.axis == 2 ? 1 : 2;
   const int uu = blockIdx.x * blockDim.x + threadIdx.x, vv = blockIdx.y;
@@ -89,7 +93,7 @@ __global__ void __launch_bounds__(128) tfsf_pre_kernel(const __grid_constant__ P
   idx[u] = p.lo[u] + uu;
   idx[v] = p.lo[v] + vv;
   const AuxTab& ax = a.aux[p.aux];
-  const long long row = a.ctrl->t - a.ctrl->t0 + ft;
+  const long long row = a.ctrl->t + a.ts - a.ctrl->t0 + ft;
   const double dt = a.dt;
   for (int w = p.lo[p.axis]; w <= p.hi[p.axis]; w++) {
     idx[p.axis] = w;
@@ -114,9 +118,9 @@ int launch_tfsf_pre(int mode, const PlainArgs& a, int ft, cudaStream_t s) {
   }
   const dim3 grid(static_cast<unsigned>((most_u + 127) / 128), static_cast<unsigned>(most_v), a.nplanes);
   switch (mode) {
-    case kTE: tfsf_pre_kernel<kTE><<<grid, 128, 0, s>>>(a, ft); break;
-    case kTM: tfsf_pre_kernel<kTM><<<grid, 128, 0, s>>>(a, ft); break;
-    default: tfsf_pre_kernel<kThreeD><<<grid, 128, 0, s>>>(a, ft); break;
+    case kTE: launch_chained(tfsf_pre_kernel<kTE>, grid, dim3(128), 0, s, a, ft); break;
+    case kTM: launch_chained(tfsf_pre_kernel<kTM>, grid, dim3(128), 0, s, a, ft); break;
+    default: launch_chained(tfsf_pre_kernel<kThreeD>, grid, dim3(128), 0, s, a, ft); break;
   }
   return 1;
 }
@@ -257,7 +261,7 @@ __device__ __forceinline__ PlainPre plain_pre_at(const PlainArgs& a, int ft, int
 template <int MODE>
 __device__ __forceinline__ PlainPre plain_pre(const PlainArgs& a, int ft, int i, int j, int k, long long c, int nz) {
   PlainPre base;
-  base.t = a.ctrl->t;
+  base.t = a.ctrl->t + a.ts;
   base.fdx[0] = a.prof[ft][0].F[i];
   base.fdx[1] = a.prof[ft][1].F[j];
   const int j0 = blockIdx.y * blockDim.y + 1;
@@ -555,6 +559,8 @@ __device__ __forceinline__ void plain_e_cell(const PlainArgs& a, int i, int j, i
 
 template <int MODE, int NP, bool HIST, int ZC, int T>
 __global__ void __launch_bounds__(T, T == 256 ? 2 : 3) plain_e_kernel(const __grid_constant__ PlainArgs a) {
+  after_previous_launch();
+  let_next_launch_start();
   extern __shared__ double smd[];
   constexpr int NS = plain_slots(MODE, 0, NP).n;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -773,6 +779,8 @@ __device__ __forceinline__ void plain_h_cell(const PlainArgs& a, int i, int j, i
 
 template <int MODE, bool HIST, int ZC, int T>
 __global__ void __launch_bounds__(T, T == 256 ? 2 : 3) plain_h_kernel(const __grid_constant__ PlainArgs a) {
+  after_previous_launch();
+  let_next_launch_start();
   extern __shared__ double smd[];
   constexpr int NS = plain_slots(MODE, 1, 0).n;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -825,7 +833,7 @@ static void plain_launch(F fn, size_t smem, const dim3& grid, const dim3& block,
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, plain_carveout(smem, ctas));
   });
-  fn<<<grid, block, smem, s>>>(a);
+  launch_chained(fn, grid, block, smem, s, a);
 }
 
 // ZC planes per thread along z (3D): the copies of plane z + 1 go into the
@@ -939,9 +947,92 @@ int launch_material_explicit(int mode, const PlainArgs& a, int ft, cudaStream_t 
 // CTA, writing Ez and Hy after every step into the tables (row 0 = the state
 // on entry). coef holds the aux CPML profile: [ft][B,Cdx,Fdx,G][L].
 // Cells 0 and L-1 see the zero ghost cells of Aux1D::Stencil1D.
-__global__ void aux_kernel(int L, double dt, double dx, double* Dz, double* Ez, double* By, double* Hy,
-                           double* psiE, double* psiH, const double* coef, const double* vals, int nvals,
-                           long long s0, int nsteps, double* Etab, double* Htab) {
+//
+// The chain of steps runs ahead of the main grid's first step, so its latency
+// counts in full: with the state and coefficients read from memory in every
+// pass, a step took 2.4 us at L = 650. Here a thread keeps the state and
+// coefficients of its C cells in registers, Ez and Hy alone pass through shared
+// memory, and a step has two barriers; the tables are written behind them.
+template <int C>
+__global__ void __launch_bounds__(1024) aux_kernel(int L, double dt, double* Dz, double* Ez, double* By, double* Hy,
+                                                   double* psiE, double* psiH, const double* coef, const double* vals,
+                                                   int nvals, long long s0, int nsteps, double* Etab, double* Htab) {
+  extern __shared__ double aux_sm[];
+  double* const E = aux_sm + 1;      // E[-1 .. L], H[-1 .. L]; the ghosts stay zero
+  double* const H = E + L + 2;
+  double D[C], B[C], pE[C], pH[C], eB[C], eC[C], eF[C], eG[C], hB[C], hC[C], hF[C], hG[C];
+  if (threadIdx.x == 0) E[-1] = E[L] = H[-1] = H[L] = 0.0;
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    const int x = threadIdx.x + c * blockDim.x;
+    if (x >= L) continue;
+    D[c] = Dz[x];
+    B[c] = By[x];
+    pE[c] = psiE[x];
+    pH[c] = psiH[x];
+    eB[c] = coef[x];
+    eC[c] = coef[L + x];
+    eF[c] = coef[2 * L + x];
+    eG[c] = coef[3 * L + x];
+    hB[c] = coef[4 * L + x];
+    hC[c] = coef[5 * L + x];
+    hF[c] = coef[6 * L + x];
+    hG[c] = coef[7 * L + x];
+    Etab[x] = E[x] = Ez[x];
+    Htab[x] = H[x] = Hy[x];
+  }
+  for (int s = 1; s <= nsteps; s++) {
+    const long long sa = s0 + s;  // aux step number
+    const double src = sa >= 1 && sa <= nvals ? vals[sa - 1] : 0.0;
+    __syncthreads();
+    // YeeUpdate<TEM,Dz>, UpdatePML<TEM,Electric,X>, VacuumUpdate E, the source
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int x = threadIdx.x + c * blockDim.x;
+      if (x >= L) continue;
+      const double diff = H[x] - H[x - 1];
+      double d = D[c] + dt * (eF[c] * diff + 0.0);
+      d += dt * pE[c] * eG[c];
+      pE[c] = eB[c] * pE[c] + eC[c] * diff;
+      D[c] = d;
+      double e = d / kEps0;
+      if (x == kAuxNpml + 5) e += src;
+      E[x] = e;
+      Etab[static_cast<long long>(s) * L + x] = e;
+    }
+    __syncthreads();
+    // YeeUpdate<TEM,By>, UpdatePML<TEM,Magnetic,X>, VacuumUpdate H
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int x = threadIdx.x + c * blockDim.x;
+      if (x >= L) continue;
+      const double diff = E[x + 1] - E[x];
+      double b = B[c] + -dt * (0.0 + -hF[c] * diff);
+      b += -dt * pH[c] * hG[c];
+      pH[c] = hB[c] * pH[c] + -hC[c] * diff;
+      B[c] = b;
+      const double h = b / kMu0;
+      H[x] = h;
+      Htab[static_cast<long long>(s) * L + x] = h;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    const int x = threadIdx.x + c * blockDim.x;
+    if (x >= L) continue;
+    Dz[x] = D[c];
+    By[x] = B[c];
+    psiE[x] = pE[c];
+    psiH[x] = pH[c];
+    Ez[x] = E[x];
+    Hy[x] = H[x];
+  }
+}
+
+// The same with the state in memory, for rows longer than the registers hold.
+__global__ void aux_long_kernel(int L, double dt, double* Dz, double* Ez, double* By, double* Hy, double* psiE,
+                                double* psiH, const double* coef, const double* vals, int nvals, long long s0,
+                                int nsteps, double* Etab, double* Htab) {
   const double* eB = coef;
   const double* eC = coef + L;
   const double* eF = coef + 2 * L;
@@ -995,7 +1086,14 @@ int launch_aux_precompute(int L, double dt, double dx, double* Dz, double* Ez, d
                           double* psiE, double* psiH, const double* coef, const double* vals, int nvals,
                           long long s0, int nsteps, double* Etab, double* Htab, cudaStream_t s) {
   (void)dx;
-  aux_kernel<<<1, 1024, 0, s>>>(L, dt, dx, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
+  const size_t smem = 2 * (static_cast<size_t>(L) + 2) * sizeof(double);
+  const int block = std::min(1024, (L + 31) / 32 * 32);
+  if (L <= 1024)
+    aux_kernel<1><<<1, block, smem, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
+  else if (L <= 2048)
+    aux_kernel<2><<<1, 1024, smem, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
+  else
+    aux_long_kernel<<<1, 1024, 0, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
   return 1;
 }
 

@@ -97,7 +97,7 @@ __device__ __forceinline__ void tfsf_cell(const FusedArgs& a, int ft, int q, con
     else if (a.bids) mid = a.bids[((k >> a.bshift) * a.nby + (j >> a.bshift)) * a.nbx + (i >> a.bshift)];
   }
   const float iemap = (ft == 0 && a.inv_eps_map) ? a.inv_eps_map[c] : 0.f;
-  const long long t = a.ctrl->t;
+  const long long t = a.ctrl->t + a.ts;
   const long long row = t - a.ctrl->t0 + (ft == 0 ? 0 : 1);
   const double inv_dx = 1.0 / a.dx;
   double corr[3] = {0.0, 0.0, 0.0};
@@ -134,6 +134,8 @@ __device__ __forceinline__ void tfsf_cell(const FusedArgs& a, int ft, int q, con
 
 template <int MODE>
 __global__ void __launch_bounds__(128) tfsf_fused_kernel(const __grid_constant__ FusedArgs a, int ft) {
+  after_previous_launch();
+  let_next_launch_start();
   const int q = blockIdx.z;
   const PlaneDev& p = a.planes[q];
   int u, v;
@@ -163,9 +165,9 @@ int launch_tfsf_fused(int mode, const FusedArgs& a, int ft, cudaStream_t s) {
   }
   const dim3 grid(static_cast<unsigned>((most_u + 127) / 128), static_cast<unsigned>(most_v), a.nplanes);
   switch (mode) {
-    case kTE: tfsf_fused_kernel<kTE><<<grid, 128, 0, s>>>(a, ft); break;
-    case kTM: tfsf_fused_kernel<kTM><<<grid, 128, 0, s>>>(a, ft); break;
-    default: tfsf_fused_kernel<kThreeD><<<grid, 128, 0, s>>>(a, ft); break;
+    case kTE: launch_chained(tfsf_fused_kernel<kTE>, grid, dim3(128), 0, s, a, ft); break;
+    case kTM: launch_chained(tfsf_fused_kernel<kTM>, grid, dim3(128), 0, s, a, ft); break;
+    default: launch_chained(tfsf_fused_kernel<kThreeD>, grid, dim3(128), 0, s, a, ft); break;
   }
   return 1;
 }
