@@ -59,14 +59,26 @@ struct NoHook {
   __device__ void operator()() const {}
 };
 
+// the first cell and row of group q of a plane, counted along the rows
+__device__ __forceinline__ void tile_group(const FusedArgs& a, int q, int& x4, int& j) {
+  const int ng = (a.nx + 3) / 4, row = q / ng;
+  x4 = 4 * (q - row * ng);
+  j = 1 + row;
+}
+
 // hook() runs after every copy of the tile has been requested, before the
 // wait for them (the one-launch kernel does its bookkeeping there).
-template <int MAXP, bool PJ, class Hook = NoHook>
+// LIN: the tile is 128 groups of plane k counted along its rows, of the
+// ceil(nx / 4) groups that a row has (bx the tile's number, by unused). A
+// lane's x neighbour is still the lane next to it: where a row starts or ends
+// between two lanes, the cells that would read across are not updated.
+template <int MAXP, bool PJ, bool LIN = false, class Hook = NoHook>
 __device__ __forceinline__ void e_tile(const FusedArgs& a, int bx, int by, int k, float4* sm, Hook hook = Hook()) {
   constexpr int kPJ = PJ ? pj_slots<MAXP>() : 0;
   const int lane = threadIdx.x, tid = threadIdx.y * 32 + lane;
-  const int x4 = bx * 128 + lane * 4;
-  const int j = 1 + by * kRowsA + threadIdx.y;
+  int x4 = bx * 128 + lane * 4;
+  int j = 1 + by * kRowsA + threadIdx.y;
+  if (LIN) tile_group(a, bx * kThreads + tid, x4, j);
   const int jl = min(j, a.ny - 2);
   const long long sy = a.pitch, sz = static_cast<long long>(a.pitch) * a.ny;
   const long long c = k * sz + jl * sy + x4;
@@ -119,22 +131,23 @@ __device__ __forceinline__ void e_tile(const FusedArgs& a, int bx, int by, int k
 // CHAIN: launched behind a kernel that may still run (launch_chained); sweeps
 // of very many CTAs are launched without (the wait alone, taken by each of
 // 882k CTAs, cost the 768^3 step 1.5%)
-template <int MAXP, int MINB, bool PJ, bool CHAIN>
+template <int MAXP, int MINB, bool PJ, bool LIN, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, MINB) staged_e_kernel(const __grid_constant__ FusedArgs a) {
   if (CHAIN) {
     after_previous_launch();
     let_next_launch_start();
   }
   extern __shared__ float4 sm[];
-  e_tile<MAXP, PJ>(a, blockIdx.x, blockIdx.y, a.kbeg + blockIdx.z, sm);
+  e_tile<MAXP, PJ, LIN>(a, blockIdx.x, blockIdx.y, a.kbeg + blockIdx.z, sm);
 }
 
 // The H update of one tile (as e_tile).
-template <bool MU>
+template <bool MU, bool LIN = false>
 __device__ __forceinline__ void h_tile(const FusedArgs& a, int bx, int by, int k, float4* sm) {
   const int lane = threadIdx.x, tid = threadIdx.y * 32 + lane;
-  const int x4 = bx * 128 + lane * 4;
-  const int j = 1 + by * kRowsA + threadIdx.y;
+  int x4 = bx * 128 + lane * 4;
+  int j = 1 + by * kRowsA + threadIdx.y;
+  if (LIN) tile_group(a, bx * kThreads + tid, x4, j);
   const int jl = min(j, a.ny - 2);
   const long long sy = a.pitch, sz = static_cast<long long>(a.pitch) * a.ny;
   const long long c = k * sz + jl * sy + x4;
@@ -169,7 +182,7 @@ __device__ __forceinline__ void h_tile(const FusedArgs& a, int bx, int by, int k
                  ez_xp3, s[7 * kThreads], s[8 * kThreads], s[9 * kThreads], px);
 }
 
-template <int MINB, bool MU, bool CHAIN>
+template <int MINB, bool MU, bool LIN, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, MINB) staged_h_kernel(const __grid_constant__ FusedArgs a) {
   if (CHAIN) {
     after_previous_launch();
@@ -177,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, MINB) staged_h_kernel(const __grid_c
   }
   extern __shared__ float4 sm[];
   // planes from the top down, as the flat H sweep
-  h_tile<MU>(a, blockIdx.x, blockIdx.y, a.kend - 1 - blockIdx.z, sm);
+  h_tile<MU, LIN>(a, blockIdx.x, blockIdx.y, a.kend - 1 - blockIdx.z, sm);
 }
 
 // The shared-memory carveout (percent of the largest) that holds `ctas` CTAs
@@ -193,8 +206,18 @@ static int carveout_for(int ctas, size_t smem) {
   return static_cast<int>(std::min<size_t>(100, (need * 100 + max_sm - 1) / max_sm));
 }
 
+// Whether to count a plane's groups along its rows instead of taking tiles of
+// 128 cells of 4 rows: where a tenth or more of the 128-cell tiles' groups
+// would lie beyond the rows' ends (nx = 132: 31 of 64). The division that
+// finds a group's row costs the full rows about 1%.
+static bool rows_padded(const FusedArgs& a) { return (a.nx + 3) / 4 * 10 <= a.pitch / 4 * 9; }
+
 static dim3 sweep_grid(const FusedArgs& a) {
   const unsigned planes = a.kend - a.kbeg;
+  if (rows_padded(a)) {
+    const long long groups = static_cast<long long>((a.nx + 3) / 4) * (a.ny - 2);
+    return dim3(static_cast<unsigned>((groups + kThreads - 1) / kThreads), 1, planes);
+  }
   return dim3(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, planes);
 }
 
@@ -215,7 +238,8 @@ static void staged_e_launch(const FusedArgs& a, cudaStream_t s) {
     launch_chained(fn, sweep_grid(a), block, smem, s, a);
   };
   const bool chain = chains(sweep_grid(a));
-  chain ? go(staged_e_kernel<MAXP, minb, PJ, true>) : go(staged_e_kernel<MAXP, minb, PJ, false>);
+  if (rows_padded(a)) chain ? go(staged_e_kernel<MAXP, minb, PJ, true, true>) : go(staged_e_kernel<MAXP, minb, PJ, true, false>);
+  else chain ? go(staged_e_kernel<MAXP, minb, PJ, false, true>) : go(staged_e_kernel<MAXP, minb, PJ, false, false>);
 }
 
 template <int MAXP>
@@ -250,7 +274,8 @@ static void staged_h_dispatch(const FusedArgs& a, cudaStream_t s) {
     launch_chained(fn, sweep_grid(a), block, smem, s, a);
   };
   const bool chain = chains(sweep_grid(a));
-  chain ? go(staged_h_kernel<8, MU, true>) : go(staged_h_kernel<8, MU, false>);
+  if (rows_padded(a)) chain ? go(staged_h_kernel<8, MU, true, true>) : go(staged_h_kernel<8, MU, true, false>);
+  else chain ? go(staged_h_kernel<8, MU, false, true>) : go(staged_h_kernel<8, MU, false, false>);
 }
 
 int launch_staged_h(const FusedArgs& a, cudaStream_t s) {
