@@ -3,8 +3,8 @@
     python -m fdtd_b200.build_lib [--force]
 
 Per-file flags:
-  kernels_plain.cu   -fmad=false: the FP64 plain method keeps every product and
-                     sum separately rounded, as the reference compiled with
+  kernels_plain.cu,  -fmad=false: the FP64 plain method keeps every product and
+  kernels_window64.cu  sum separately rounded, as the reference compiled with
                      -ffp-contract=off.
   fdtd_capi.cu       host code with -ffp-contract=off (CPML / material
                      coefficient set-up in the reference's rounding).
@@ -33,11 +33,12 @@ SOURCES = {
     "kernels_tfsf.cu": [],
     "kernels_batch.cu": [],
     "kernels_window.cu": [],
+    "kernels_window64.cu": ["-fmad=false"],
     "kernels_common.cu": [],
     "kernels_adjoint.cu": [],
     "fdtd_capi.cu": [],
 }
-HEADERS = ["internal.h", "fused3d_common.cuh", "pairs.cuh", os.path.join("..", "..", "include", "fdtd_b200.h")]
+HEADERS = ["internal.h", "fused3d_common.cuh", "pairs.cuh", "plain_tfsf.cuh", "quotient.cuh", os.path.join("..", "..", "include", "fdtd_b200.h")]
 
 
 def _newer(target: str, deps) -> bool:

@@ -215,11 +215,13 @@ struct fdtd_grid {
   int scheme = 1;     // time policy of the curl updates: 1 BD1, 3 BD3, 4 BD4
   void* hist[2][3][3]{};  // FP64 flux history [D|B][level][comp] of BD3/BD4
   int sweep_kind = FDTD_SWEEP_AUTO;
-  // temporal blocking of 2D FP32 grids: the second copy of the state (fields,
+  // temporal blocking of 2D grids: the second copy of the state (fields,
   // CPML integrators, soft sources' last values) and 1/eps per cell, the
   // kernel's arguments and the version they were made for
   void* win_block = nullptr;  // one allocation for all of it
   WinArgs win{};
+  Win64Args win64{};
+  double* win_tfsf = nullptr;  // FP64: the TFSF corrections of a stretch of steps
   long long win_version = -1;
   bool win_ok = false;
   TmaState* tma = nullptr;
@@ -716,6 +718,7 @@ PlainArgs plain_args(fdtd_grid* g) {
   a.mats = static_cast<const MatF64*>(g->d_mats);
   a.eps_map = static_cast<const double*>(g->d_eps_map);
   a.tfsf_pre = g->d_tfsf_pre;
+  a.tfsf_cells = g->tfsf_cells;
   a.dispersive = g->max_poles;
   a.all_dispersive = g->mats.empty() ? 0 : 1;
   for (auto& m : g->mats)
@@ -812,15 +815,22 @@ void window_arrays(const fdtd_grid* g, void* (&f)[3], void* (&psi)[4]) {
   psi[3] = g->psi[1][te ? 2 : 1][0];
 }
 
-// What the windows do not cover keeps the launches per half step: poles,
-// mu_r, TFSF planes, boundary conditions, DFT of surface quantities, more
+// What the windows do not cover keeps the launches per half step: poles (FP32),
+// mu_r, TFSF planes (FP32), BD3/BD4, boundary conditions, DFT of surface quantities, more
 // boxes or regions than a window lists, and a sweep kernel set by hand.
 bool window_wanted(const fdtd_grid* g) {
-  if (!g->f32 || g->d.mode == kThreeD || g->sweep_kind != FDTD_SWEEP_AUTO) return false;
-  if (g->max_poles != 0 || g->bcs.n > 0 || !g->planes.empty()) return false;
+  if (g->d.mode == kThreeD || g->sweep_kind != FDTD_SWEEP_AUTO || g->bcs.n > 0) return false;
   if (g->boxes.size() > static_cast<size_t>(kWinMaxBoxes)) return false;
+  if (g->f32) {
+    if (g->max_poles != 0 || !g->planes.empty()) return false;
+  } else {
+    // FP64 windows take TFSF planes, and one pole (TE) or two (TM); what acts in
+    // one is listed in 32 entries (a plane is two)
+    if (g->scheme != 1 || g->max_poles * (g->d.mode == kTE ? 2 : 1) > kWin64Poles || g->mats.size() > 65535) return false;
+    if (2 * g->planes.size() + g->srcs.size() + g->boxes.size() > 32) return false;
+  }
   for (const auto& m : g->mats)
-    if (m.mu_r != 1.0) return false;
+    if (m.mu_r != (g->f32 ? 1.0 : g->mats[0].mu_r)) return false;
   int n[2] = {0, 0};
   for (const auto& r : g->dfts) {
     if (r.comp >= 6) return false;
@@ -889,6 +899,8 @@ bool window_uniform(const fdtd_grid* g) {
 // Lays out the second copy of the state and 1/eps of a grid that takes its
 // steps in windows, again after any change to it. A grid whose second copy
 // does not fit in device memory keeps the launches per half step.
+int ensure_window64(fdtd_grid* g);
+
 int ensure_window(fdtd_grid* g) {
   if (g->win_version == g->version) return FDTD_OK;
   g->win_ok = false;
@@ -896,6 +908,7 @@ int ensure_window(fdtd_grid* g) {
     g->win_version = g->version;
     return FDTD_OK;
   }
+  if (!g->f32) return ensure_window64(g);
   void *f[3], *psi[4];
   window_arrays(g, f, psi);
   // the parts of the block: fields, integrators, src_last, 1/eps
@@ -934,6 +947,113 @@ int ensure_window(fdtd_grid* g) {
   return FDTD_OK;
 }
 
+// the FP64 grids' part of it
+int ensure_window64(fdtd_grid* g) {
+  const bool te = g->d.mode == kTE;
+  const int ne = te ? 2 : 1, nh = te ? 1 : 2, np = g->max_poles;
+  void *f[3], *psi[4];
+  window_arrays(g, f, psi);
+  // the parts of the block: D, E (2 each), B, H (2 each), integrators, P and
+  // J, the divisors and poles of the cells, the TFSF corrections
+  std::vector<void*> own;
+  for (int q = 0; q < 2; q++) {
+    const int ce = te ? q : 2, ch = te ? 2 : q;
+    own.push_back(q < ne ? g->D[ce] : nullptr);
+    own.push_back(q < ne ? g->E[ce] : nullptr);
+    own.push_back(q < nh ? g->B[ch] : nullptr);
+    own.push_back(q < nh ? g->H[ch] : nullptr);
+  }
+  for (auto* p : psi) own.push_back(p);
+  for (int q = 0; q < ne; q++)
+    for (int pole = 0; pole < np; pole++) {
+      own.push_back(g->P[pole][te ? q : 2]);
+      own.push_back(g->J[pole][te ? q : 2]);
+    }
+  std::vector<size_t> at;
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    at.push_back(total);
+    total += (bytes + 255) / 256 * 256;
+  };
+  const size_t cells = static_cast<size_t>(field_elems(g));
+  for (auto* p : own) part(p ? g->sizes[p] : 0);
+  part(window_uniform(g) ? 0 : cells * sizeof(double));
+  part(np > 0 ? cells * sizeof(unsigned short) : 0);
+  part(static_cast<size_t>(g->tfsf_cells) * 3 * 2 * kDftChunk * sizeof(double));
+  if (!g->win_block || g->sizes[g->win_block] != total) {
+    dfree(g, g->win_block);
+    const int rc = dalloc(g, &g->win_block, total);
+    if (rc) {
+      g->win_version = g->version;
+      return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
+    }
+  }
+  char* const b = static_cast<char*>(g->win_block);
+  auto twin = [&](size_t q) { return own[q] ? reinterpret_cast<double*>(b + at[q]) : nullptr; };
+  const PlainArgs pa = plain_args(g);
+  const WinArgs wa = window_args(g);  // the parts that do not depend on the precision
+  Win64Args& w = g->win64;
+  memset(&w, 0, sizeof(w));
+  w.mode = g->d.mode;
+  w.nx = g->n[0];
+  w.ny = g->n[1];
+  w.dt = pa.dt;
+  w.den_h = g->mats[0].mu_r * kMu0;
+  w.rden_h = 1.0 / w.den_h;
+  for (int x = 0; x < 2; x++) {
+    w.pml[x] = wa.pml[x];
+    w.slab[x] = wa.slab[x];
+    for (int q = 0; q < 2; q++) w.plain[x][q] = wa.plain[x][q];
+    for (int h = 0; h < 2; h++) w.prof[h][x] = pa.prof[h][x];
+  }
+  for (int q = 0; q < 2; q++) {
+    double** sets[4] = {&w.D[0][q], &w.E[0][q], &w.B[0][q], &w.H[0][q]};
+    double** tsets[4] = {&w.D[1][q], &w.E[1][q], &w.B[1][q], &w.H[1][q]};
+    for (int k = 0; k < 4; k++) {
+      *sets[k] = static_cast<double*>(own[4 * q + k]);
+      *tsets[k] = twin(4 * q + k);
+    }
+  }
+  for (int q = 0; q < 4; q++) {
+    w.psi[0][q] = static_cast<double*>(own[8 + q]);
+    w.psi[1][q] = twin(8 + q);
+  }
+  for (int q = 0; q < 2 * np * ne; q++) {
+    w.pj[0][q] = static_cast<double*>(own[12 + q]);
+    w.pj[1][q] = twin(12 + q);
+  }
+  const size_t rest = own.size();
+  w.den0 = (g->mats[0].kind == FDTD_VACUUM ? 1.0 : g->mats[0].eps_inf) * kEps0;
+  w.rden0 = 1.0 / w.den0;
+  double* const den = window_uniform(g) ? nullptr : reinterpret_cast<double*>(b + at[rest]);
+  unsigned short* const disp = np > 0 ? reinterpret_cast<unsigned short*>(b + at[rest + 1]) : nullptr;
+  w.den = den;
+  w.disp = disp;
+  w.np = np;
+  w.mats = pa.mats;
+  if (den || disp) g->launches += launch_window64_cells(pa, den, disp, g->stream);
+  w.nsrc = wa.nsrc;
+  w.nbox = wa.nbox;
+  w.nplanes = pa.nplanes;
+  for (int q = 0; q < wa.nsrc; q++) w.src[q] = wa.src[q];
+  for (int q = 0; q < wa.nbox; q++) w.box[q] = wa.box[q];
+  for (int q = 0; q < pa.nplanes; q++) w.planes[q] = pa.planes[q];
+  w.tfsf_cells = g->tfsf_cells;
+  g->win_tfsf = reinterpret_cast<double*>(b + at[rest + 2]);
+  w.tfsf = g->win_tfsf;
+  for (int ph = 0; ph < 2; ph++) {
+    w.nreg[ph] = g->ndft[ph];
+    w.reg[ph] = g->d_dft[ph];
+    w.dft_buf[ph] = static_cast<double*>(g->d_dft_buf[ph]);
+    w.dft_pts[ph] = g->dft_pts[ph];
+  }
+  w.ctrl = g->ctrl;
+  CK(cudaStreamSynchronize(g->stream));  // as for the FP32 windows
+  g->win_version = g->version;
+  g->win_ok = true;
+  return FDTD_OK;
+}
+
 // Steps per launch and rows per window: the pair with the least modelled time
 // of a step. A launch takes from its predecessor's end about 4 us + 1.05 us a
 // step with windows of 32 rows, 8 us + 1.5 us a step with 64 (measured at
@@ -957,6 +1077,24 @@ int window_steps(int nx, int ny, int* rows) {
         *rows = R;
       }
     }
+  return best;
+}
+
+// Steps per launch of FP64 windows, one per SM: a round of windows takes about
+// 10 us + 3 us a step (256 x 256: 21 us at 4 steps, 28 at 6, 33 at 8; 600 x 450
+// with poles and TFSF, two rounds at 5 and 6 steps: 57 and 63, three at 8: 116).
+int window64_steps(int nx, int ny) {
+  int best = 8;
+  double least = 1e30;
+  for (int L : {16, 14, 12, 10, 8, 6}) {
+    const int T = (kGraphSteps + L - 1) / L;
+    const double rounds = std::ceil(window64_count(nx, ny, T) / 148.0);
+    const double t = rounds * (10.0 + 3.0 * T) * L;
+    if (t < least) {
+      least = t;
+      best = T;
+    }
+  }
   return best;
 }
 
@@ -1578,11 +1716,14 @@ int fdtd_prepare(fdtd_grid* g) try {
   }
   // the step graph too (its capture launches nothing), so that the first
   // call of kGraphSteps or more steps replays it at once
-  rc = ensure_window(g);
-  if (rc) return rc;
-  if (g->use_graphs && g->next_half == 0 && !g->half_split) {
+  const bool graph = g->use_graphs && g->next_half == 0 && !g->half_split;
+  if (graph) {
     rc = ensure_aux_tables(g, kGraphSteps);
     if (rc) return rc;
+  }
+  rc = ensure_window(g);
+  if (rc) return rc;
+  if (graph) {
     if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
     rc = ensure_step_graph(g, g->stream);
     if (rc) return rc;
@@ -1741,7 +1882,9 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
   if (adj) adjoint_capture_args(adj, wa);
   const bool dft = !g->dfts.empty();
   int rows = kWinRows;
-  const int T = window_steps(g->n[0], g->n[1], &rows);
+  const int T = g->f32 ? window_steps(g->n[0], g->n[1], &rows) : window64_steps(g->n[0], g->n[1]);
+  PlainArgs pa;
+  if (!g->planes.empty()) pa = plain_args(g);
   for (int done = 0; done < nsteps;) {
     const int n = std::min(nsteps - done, kDftChunk - (dft ? g->dft_pending : 0));
     if (n == 1) {
@@ -1752,10 +1895,12 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
       continue;
     }
     const int L = 2 * ((n + 2 * T - 1) / (2 * T));
+    if (!g->planes.empty()) g->launches += launch_tfsf_table(g->d.mode, pa, n, g->win_tfsf, s);
     for (int q = 0; q < L; q++) {
       const int at = static_cast<int>(static_cast<long long>(n) * q / L);
       const int t = static_cast<int>(static_cast<long long>(n) * (q + 1) / L) - at;
-      g->launches += launch_window(g->d.mode, wa, rows, t, at, q & 1, g->dft_pending + at, s);
+      g->launches += g->f32 ? launch_window(g->d.mode, wa, rows, t, at, q & 1, g->dft_pending + at, s)
+                            : launch_window64(g->d.mode, g->win64, t, at, q & 1, g->dft_pending + at, s);
     }
     g->launches += launch_steps_advance(g->ctrl, n, s);
     if (dft) {
@@ -1786,6 +1931,8 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
       if (prc) return prc;
       CK(cudaStreamSynchronize(g->stream));
     }
+    prc = ensure_aux_tables(g, nsteps);
+    if (prc) return prc;
     prc = ensure_window(g);
     if (prc) return prc;
   }
@@ -1799,10 +1946,6 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     CK(cudaEventDestroy(ev));
   }
   // TFSF: precompute the aux grids' Ez/Hy for this chunk of steps
-  {
-    const int rc = ensure_aux_tables(g, nsteps);
-    if (rc) return rc;
-  }
   for (auto& a : g->auxes) {
     double* st = a.d_state;
     const int L = a.L;

@@ -221,6 +221,7 @@ struct PlainArgs {
   // the half step's TFSF corrections of every plane cell ([off + cell][3]),
   // formed before each sweep by launch_tfsf_pre
   double* tfsf_pre;
+  long long tfsf_cells;  // cells of all planes
 };
 
 struct FusedArgs {
@@ -348,6 +349,43 @@ struct AdjArgs {
   double* grad;                     // dJ/deps_r, design box order
   const Control* ctrl;              // the grid's step counter
 };
+
+// The same of a 2D FP64 grid (kernels_window64.cu): D, E, B, H in the reference's
+// form; E components Ex, Ey (TE) or Ez, H components Hz or Hx, Hy
+struct Win64Args {
+  int mode, nx, ny;
+  int pml[2];
+  Slab slab[2];
+  int plain[2][2];
+  double dt, den_h, rden_h;     // rden: the correctly rounded reciprocals
+  double *D[2][2], *E[2][2], *B[2][2], *H[2][2];
+  double* psi[2][4];
+  double* pj[2][8];             // per E component: P, J of the first pole, of the second
+  const double* den;            // per cell, or null: den0 everywhere
+  double den0, rden0;
+  const unsigned short* disp;   // 1 + the material of a cell with poles, 0 without; np the most poles
+  int np;
+  const MatF64* mats;
+  Prof<double> prof[2][2];
+  int nsrc, nbox, nplanes;
+  SourceDev src[kMaxSources];
+  WinBox box[kWinMaxBoxes];
+  PlaneDev planes[kMaxPlanes];
+  const double* tfsf;           // [step][half][plane cell][component]
+  long long tfsf_cells;
+  int nreg[2];
+  const DftRegionDev* reg[2];
+  double* dft_buf[2];
+  long long dft_pts[2];
+  const Control* ctrl;
+};
+// poles times E components that a window's shared memory holds P and J of
+constexpr int kWin64Poles = 2;
+int window64_count(int nx, int ny, int T);
+int launch_window64(int mode, const Win64Args& a, int T, int s, int from, int slot, cudaStream_t st);
+// the TFSF corrections of the nsteps steps from the counter on
+int launch_tfsf_table(int mode, const PlainArgs& a, int nsteps, double* out, cudaStream_t s);
+int launch_window64_cells(const PlainArgs& a, double* den, unsigned short* disp, cudaStream_t s);
 
 // The reversed steps in windows: what AdjArgs holds, on two copies of the
 // adjoint state

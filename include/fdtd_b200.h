@@ -214,13 +214,15 @@ int fdtd_dft_read(fdtd_grid* g, int handle, double* out);
 /* Advance nsteps full time steps on `stream` (a cudaStream_t, or NULL for the
  * handle's stream). Returns once the work is enqueued. */
 int fdtd_step(fdtd_grid* g, int nsteps, void* stream);
-/* 2D FP32 grids of non-dispersive materials with mu_r = 1, without TFSF
- * planes, boundary conditions or DFT of surface quantities take calls of two
- * steps or more in windows: several steps per launch, from one copy of the
- * state into another (the grid holds a second copy of its fields and CPML
- * integrators, and 1/eps per cell). Results are those of one launch per half
- * step, which fdtd_set_sweep_kernel(g, FDTD_SWEEP_REGS) brings back, and
- * which a grid keeps whose second copy finds no device memory. */
+/* 2D grids take calls of two steps or more in windows: several steps per
+ * launch, from one copy of the state into another (the grid holds a second
+ * copy of what a step changes, and per-cell material factors). FP32 grids do
+ * without poles, mu_r != 1 and TFSF planes; FP64 grids with one mu_r, BD1, at
+ * most one pole (TE) or two (TM) and 32 of sources, boxes and twice the TFSF
+ * planes; both without boundary conditions and DFT of surface quantities.
+ * Results are those of one launch per half step, which
+ * fdtd_set_sweep_kernel(g, FDTD_SWEEP_REGS) brings back, and which a grid
+ * keeps whose second copy finds no device memory. */
 /* Half a time step: phase 0 = the E half (curl of H, CPML, materials,
  * sources, TFSF, E-phase DFT sample; it also advances the TFSF aux grids one
  * step), phase 1 = the H half, which completes the step. The halves must

@@ -1,4 +1,4 @@
-"""2D FP32 grids stepped in windows (several steps per launch) against the
+"""2D grids stepped in windows (several steps per launch) against the
 same grid stepped with one launch per half step (the sweep kernel set by
 hand): the arithmetic per cell is the same, so every stored value is equal.
 Extents at and around the windows' edges (64 columns, 32 and 64 rows, and the
@@ -86,3 +86,46 @@ def test_windows_on_a_caller_stream_without_graphs(fdtd):
         out.append([g.get(n) for n in ("Ex", "Ey", "Hz")] + [g.dft(0)])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def _problem64(mode, nx, ny, seed, poles):
+    """The same with TFSF planes where they fit, and materials with poles."""
+    p = _problem(mode, nx, ny, seed)
+    dt = p.dt
+    if poles:
+        p.materials[1] = P.Material.drude(1.0, 0.25 / dt, 0.02 / dt)
+        lor = [(1.2, 0.1 / dt, 0.01 / dt), (0.6, 0.2 / dt, 0.02 / dt)][:poles]
+        p.materials[2] = P.Material.lorentz(1.5, lor)
+        rng = np.random.default_rng(seed)
+        p.ids = (rng.integers(0, 3, size=(1, ny, nx)) * (rng.random((1, ny, nx)) < 0.2)).astype(np.uint8)
+    if min(nx, ny) >= 30:
+        k = (np.cos(0.3), np.sin(0.3), 0.0)
+        pe, ph = P.ref_te_polarisation(k) if mode == P.TE else P.ref_tm_polarisation(k)
+        p.tfsf = P.TFSF(2 * max(nx, ny), P.gaussian_pulse(120, 30, 8, offset=1.0), (nx / 2, ny / 2, 0.0), k, pe, ph,
+                        P.tfsf_box_planes(mode, (11, 10), (nx - 12, ny - 11)))
+    return p
+
+
+@pytest.mark.parametrize("mode", [P.TE, P.TM], ids=["te", "tm"])
+@pytest.mark.parametrize("nx,ny,poles", [(3, 3, 0), (64, 32, 0), (65, 33, 1), (31, 64, 2), (113, 47, 0), (112, 48, 1),
+                                         (200, 131, 2), (410, 300, 0)])
+def test_fp64_windows_equal_the_half_step_launches(fdtd, mode, nx, ny, poles):
+    p = _problem64(mode, nx, ny, nx + ny, poles)
+    E, H, D, B = mode_fields(mode)
+    names = E + H + D + B + ["Px", "Py", "Pz", "Jx", "Jy", "Jz"] + list(fdtd.PSI_NAMES)
+    out = []
+    for kind in ("auto", "regs"):
+        g = fdtd.Grid.from_problem(p, "f64")
+        g.set_sweep_kernel(kind)
+        for n in (1, 2, 3, 13, 64, 71):
+            g.step(n)
+        vals = []
+        for n in names:
+            try:
+                vals.append(g.get(n))
+            except fdtd.FdtdError:
+                pass
+        out.append(vals + [g.dft(h) for h in g.dft_handles])
+    assert any(np.any(v) for v in out[0])
+    for q, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a, b), (q, float(np.abs(a - b).max()))
