@@ -20,6 +20,7 @@
 
 #include "../../include/fdtd_b200.h"
 #include "internal.h"
+#include "quotient.cuh"
 
 using namespace fdtdb;
 
@@ -999,7 +1000,7 @@ int ensure_window64(fdtd_grid* g) {
   w.ny = g->n[1];
   w.dt = pa.dt;
   w.den_h = g->mats[0].mu_r * kMu0;
-  w.rden_h = 1.0 / w.den_h;
+  w.rden_h = quotient_reciprocal(w.den_h);
   for (int x = 0; x < 2; x++) {
     w.pml[x] = wa.pml[x];
     w.slab[x] = wa.slab[x];
@@ -1024,7 +1025,7 @@ int ensure_window64(fdtd_grid* g) {
   }
   const size_t rest = own.size();
   w.den0 = (g->mats[0].kind == FDTD_VACUUM ? 1.0 : g->mats[0].eps_inf) * kEps0;
-  w.rden0 = 1.0 / w.den0;
+  w.rden0 = quotient_reciprocal(w.den0);
   double* const den = window_uniform(g) ? nullptr : reinterpret_cast<double*>(b + at[rest]);
   unsigned short* const disp = np > 0 ? reinterpret_cast<unsigned short*>(b + at[rest + 1]) : nullptr;
   w.den = den;

@@ -357,7 +357,7 @@ struct Win64Args {
   int pml[2];
   Slab slab[2];
   int plain[2][2];
-  double dt, den_h, rden_h;     // rden: the correctly rounded reciprocals
+  double dt, den_h, rden_h;     // rden: the reciprocals (quotient_reciprocal)
   double *D[2][2], *E[2][2], *B[2][2], *H[2][2];
   double* psi[2][4];
   double* pj[2][8];             // per E component: P, J of the first pole, of the second

@@ -254,7 +254,7 @@ __device__ __forceinline__ void window64_run(const Win64Args& a, Shared64& sh, d
     }
     const double den = a.den ? (here ? a.den[at] : 1.0) : a.den0;
     den_at[c] = den;
-    den_at[c + kCells] = a.den ? 1.0 / den : a.rden0;
+    den_at[c + kCells] = a.den ? quotient_reciprocal(den) : a.rden0;
   }
   const bool has_poles = GEN && __any_sync(kAll, (mid[0] | mid[1]) != 0);
   int xs[2] = {-1, -1}, ys = -1;
@@ -326,9 +326,10 @@ __device__ __forceinline__ void window64_run(const Win64Args& a, Shared64& sh, d
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         const double fx = c ? fx1 : fx0;
+        // (+ 0.0: the term of the absent component, which turns -0 into +0)
         if (TE) {
-          d[0][c] = D[0][c] + dt * (fy * dfy[c]);
-          d[NE - 1][c] = D[NE - 1][c] + dt * (-fx * dfx[c]);
+          d[0][c] = D[0][c] + dt * (fy * dfy[c] + 0.0);
+          d[NE - 1][c] = D[NE - 1][c] + dt * (-fx * dfx[c] + 0.0);
         } else {
           d[0][c] = D[0][c] + dt * (fx * dfx[c] + -fy * dfy[c]);
         }
@@ -345,8 +346,8 @@ __device__ __forceinline__ void window64_run(const Win64Args& a, Shared64& sh, d
         if (has_x) pml_x(1, 0, dt, TE ? -1.0 : 1.0, dfx, d[NE - 1]);
         if (has_y) pml_y(0, 0, dt, TE ? 1.0 : -1.0, dfy, d[0]);
       }
-      bool easy = true;
       const double2 den = *reinterpret_cast<const double2*>(den_at), rden = *reinterpret_cast<const double2*>(den_at + kCells);
+      bool easy = quotient_by(rden.x) && quotient_by(rden.y);
 #pragma unroll
       for (int q = 0; q < NE; q++)
 #pragma unroll
@@ -398,8 +399,8 @@ __device__ __forceinline__ void window64_run(const Win64Args& a, Shared64& sh, d
         if (TE) {
           b[0][c] = B[0][c] + -dt * (fx * dfx[c] + -fy * dfy[c]);
         } else {
-          b[0][c] = B[0][c] + -dt * (fy * dfy[c]);
-          b[NH - 1][c] = B[NH - 1][c] + -dt * (-fx * dfx[c]);
+          b[0][c] = B[0][c] + -dt * (fy * dfy[c] + 0.0);
+          b[NH - 1][c] = B[NH - 1][c] + -dt * (-fx * dfx[c] + 0.0);
         }
       }
       if (GEN) {
@@ -413,7 +414,7 @@ __device__ __forceinline__ void window64_run(const Win64Args& a, Shared64& sh, d
         if (has_x) pml_x(3, 1, -dt, TE ? 1.0 : -1.0, dfx, b[NH - 1]);
         if (has_y) pml_y(2, 1, -dt, TE ? -1.0 : 1.0, dfy, b[0]);
       }
-      bool easy = true;
+      bool easy = quotient_by(a.rden_h);
 #pragma unroll
       for (int q = 0; q < NH; q++)
 #pragma unroll

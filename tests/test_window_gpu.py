@@ -129,3 +129,30 @@ def test_fp64_windows_equal_the_half_step_launches(fdtd, mode, nx, ny, poles):
     assert any(np.any(v) for v in out[0])
     for q, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a, b), (q, float(np.abs(a - b).max()))
+
+
+@pytest.mark.parametrize("mode", [P.TE, P.TM], ids=["te", "tm"])
+@pytest.mark.parametrize("eps,mu_r", [(np.inf, 1.0), (1e60, 1.0), (1e-25, 1e-25), (2.0, np.inf), (2.0, 1e60)])
+def test_fp64_windows_with_divisors_at_the_ends_of_the_range(fdtd, mode, eps, mu_r):
+    """Divisors whose reciprocals do not give the quotient, and zeros of either
+    sign: every stored value, the zeros' signs too, as the half-step launches'."""
+    nx, ny = 70, 41
+    p = _problem64(mode, nx, ny, 5, 0)
+    p.tfsf = None
+    p.materials = [P.Material.constant(1.5, mu_r), P.Material.constant(eps, mu_r)]
+    p.ids = (np.indices((1, ny, nx))[2] % 7 == 3).astype(np.uint8)
+    E, H, D, B = mode_fields(mode)
+    rng = np.random.default_rng(1)
+    start = {n: np.where(rng.random((1, ny, nx)) < 0.5, -0.0, rng.normal(size=(1, ny, nx)) * 1e-12) for n in D + B}
+    out = []
+    for kind in ("auto", "regs"):
+        g = fdtd.Grid.from_problem(p, "f64")
+        g.set_sweep_kernel(kind)
+        for n, v in start.items():
+            g.set(n, v)
+        g.step(4)
+        out.append([g.get(n) for n in E + H + D + B])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b, equal_nan=True)
+        ok = ~np.isnan(a)
+        assert np.array_equal(np.signbit(a[ok]), np.signbit(b[ok]))
