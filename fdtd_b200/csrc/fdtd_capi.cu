@@ -222,7 +222,8 @@ struct fdtd_grid {
   void* win_block = nullptr;  // one allocation for all of it
   WinArgs win{};
   Win64Args win64{};
-  double* win_tfsf = nullptr;  // FP64: the TFSF corrections of a stretch of steps
+  void* win_tfsf = nullptr;  // the TFSF corrections of a stretch of steps
+  WinExt win_ext;            // FP32: what poles and TFSF planes need
   long long win_version = -1;
   bool win_ok = false;
   TmaState* tma = nullptr;
@@ -816,14 +817,14 @@ void window_arrays(const fdtd_grid* g, void* (&f)[3], void* (&psi)[4]) {
   psi[3] = g->psi[1][te ? 2 : 1][0];
 }
 
-// What the windows do not cover keeps the launches per half step: poles (FP32),
-// mu_r, TFSF planes (FP32), BD3/BD4, boundary conditions, DFT of surface quantities, more
+// What the windows do not cover keeps the launches per half step: more poles than
+// fit in shared memory (FP64), mu_r, BD3/BD4, boundary conditions, DFT of surface quantities, more
 // boxes or regions than a window lists, and a sweep kernel set by hand.
 bool window_wanted(const fdtd_grid* g) {
   if (g->d.mode == kThreeD || g->sweep_kind != FDTD_SWEEP_AUTO || g->bcs.n > 0) return false;
   if (g->boxes.size() > static_cast<size_t>(kWinMaxBoxes)) return false;
   if (g->f32) {
-    if (g->max_poles != 0 || !g->planes.empty()) return false;
+    if (g->max_poles != 0 && g->mats.size() > 16384) return false;  // a cell's poles and material in 16 bits
   } else {
     // FP64 windows take TFSF planes, and one pole (TE) or two (TM); what acts in
     // one is listed in 32 entries (a plane is two)
@@ -921,6 +922,23 @@ int ensure_window(fdtd_grid* g) {
   };
   for (int q = 0; q < 8; q++) part(q, own[q] ? g->sizes[own[q]] : 0);
   part(8, window_uniform(g) ? 0 : static_cast<size_t>(field_elems(g)) * sizeof(float));
+  // poles and TFSF: J and P, the cells' materials, the corrections
+  const bool te = g->d.mode == kTE;
+  const int ne = te ? 2 : 1, np = std::abs(g->max_poles), per = g->max_poles < 0 ? 1 : 2;
+  std::vector<void*> pj;
+  for (int q = 0; q < ne; q++)
+    for (int p = 0; p < np; p++) {
+      pj.push_back(g->J[p][te ? q : 2]);
+      if (per == 2) pj.push_back(g->P[p][te ? q : 2]);
+    }
+  std::vector<size_t> more;
+  auto extra = [&](size_t bytes) {
+    more.push_back(total);
+    total += (bytes + 255) / 256 * 256;
+  };
+  for (auto* p : pj) extra(g->sizes[p]);
+  extra(np > 0 ? static_cast<size_t>(field_elems(g)) * sizeof(unsigned short) : 0);
+  extra(static_cast<size_t>(g->tfsf_cells) * 2 * kDftChunk * sizeof(float));
   if (!g->win_block || g->sizes[g->win_block] != total) {
     dfree(g, g->win_block);
     const int rc = dalloc(g, &g->win_block, total);
@@ -940,6 +958,27 @@ int ensure_window(fdtd_grid* g) {
     g->win.ie = ie;
     g->launches += launch_adjoint_inv_eps(fused_args(g), ie, g->stream);
   }
+  const FusedArgs fa = fused_args(g);
+  WinExt& x = g->win_ext;
+  memset(&x, 0, sizeof(x));
+  x.np = np;
+  x.per = per;
+  for (size_t q = 0; q < pj.size(); q++) {
+    x.pj[0][q] = static_cast<float*>(pj[q]);
+    x.pj[1][q] = reinterpret_cast<float*>(b + more[q]);
+  }
+  unsigned short* const disp = reinterpret_cast<unsigned short*>(b + more[pj.size()]);
+  if (np > 0) g->launches += launch_window_cells(fa, disp, g->stream);
+  x.disp = disp;
+  x.mats = fa.mats;
+  x.nplanes = fa.nplanes;
+  for (int q = 0; q < fa.nplanes; q++) {
+    const PlaneDev& p = fa.planes[q];
+    x.plane[q] = WinPlane{p.axis, {p.lo[0], p.lo[1]}, {p.hi[0], p.hi[1]}, p.off};
+  }
+  g->win_tfsf = b + more[pj.size() + 1];
+  x.tfsf = static_cast<const float*>(g->win_tfsf);
+  x.tfsf_cells = g->tfsf_cells;
   // the windows read what was set up here before they wait for the launch
   // ahead of them (launch_chained): it is all in place once this returns
   CK(cudaStreamSynchronize(g->stream));
@@ -1040,8 +1079,8 @@ int ensure_window64(fdtd_grid* g) {
   for (int q = 0; q < wa.nbox; q++) w.box[q] = wa.box[q];
   for (int q = 0; q < pa.nplanes; q++) w.planes[q] = pa.planes[q];
   w.tfsf_cells = g->tfsf_cells;
-  g->win_tfsf = reinterpret_cast<double*>(b + at[rest + 2]);
-  w.tfsf = g->win_tfsf;
+  g->win_tfsf = b + at[rest + 2];
+  w.tfsf = static_cast<const double*>(g->win_tfsf);
   for (int ph = 0; ph < 2; ph++) {
     w.nreg[ph] = g->ndft[ph];
     w.reg[ph] = g->d_dft[ph];
@@ -1061,10 +1100,11 @@ int ensure_window64(fdtd_grid* g) {
 // 317 x 233), and each further round of windows (two per SM) 5 and 11.5 us +
 // 0.1 us a step (3001 x 2047: 32 rows 19.7 us a step at 8 steps, 64 rows 20.9
 // at 4, 14.3 at 8, 14.2 at 12, 16.3 at 16).
-int window_steps(int nx, int ny, int* rows) {
+int window_steps(int nx, int ny, int* rows, int most_rows = kWinRows) {
   int best = 8;
   double least = 1e30;
   for (int R : {32, 64})
+    if (R <= most_rows)
     for (int L : {16, 12, 8, 6, 4}) {
       const int T = (kGraphSteps + L - 1) / L;
       if (4 * T > R + 16) continue;
@@ -1883,9 +1923,17 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
   if (adj) adjoint_capture_args(adj, wa);
   const bool dft = !g->dfts.empty();
   int rows = kWinRows;
-  const int T = g->f32 ? window_steps(g->n[0], g->n[1], &rows) : window64_steps(g->n[0], g->n[1]);
+  // with Lorentz poles a window of 64 rows is more than an SM's shared memory;
+  // with Drude poles one fits instead of two and is still the faster (3000 x
+  // 2000: 22.2 us a step against 25.5 in windows of 32 rows)
+  const int most = g->f32 && g->max_poles > 0 ? 32 : kWinRows;
+  const int T = g->f32 ? window_steps(g->n[0], g->n[1], &rows, most) : window64_steps(g->n[0], g->n[1]);
   PlainArgs pa;
-  if (!g->planes.empty()) pa = plain_args(g);
+  FusedArgs fa;
+  const bool tfsf = !g->planes.empty();
+  if (tfsf && !g->f32) pa = plain_args(g);
+  if (tfsf && g->f32) fa = fused_args(g);
+  const WinExt* const ext = g->f32 && (tfsf || g->max_poles != 0) ? &g->win_ext : nullptr;
   for (int done = 0; done < nsteps;) {
     const int n = std::min(nsteps - done, kDftChunk - (dft ? g->dft_pending : 0));
     if (n == 1) {
@@ -1896,11 +1944,12 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
       continue;
     }
     const int L = 2 * ((n + 2 * T - 1) / (2 * T));
-    if (!g->planes.empty()) g->launches += launch_tfsf_table(g->d.mode, pa, n, g->win_tfsf, s);
+    if (tfsf && g->f32) g->launches += launch_tfsf_fused_table(g->d.mode, fa, n, g->tfsf_cells, static_cast<float*>(g->win_tfsf), s);
+    if (tfsf && !g->f32) g->launches += launch_tfsf_table(g->d.mode, pa, n, static_cast<double*>(g->win_tfsf), s);
     for (int q = 0; q < L; q++) {
       const int at = static_cast<int>(static_cast<long long>(n) * q / L);
       const int t = static_cast<int>(static_cast<long long>(n) * (q + 1) / L) - at;
-      g->launches += g->f32 ? launch_window(g->d.mode, wa, rows, t, at, q & 1, g->dft_pending + at, s)
+      g->launches += g->f32 ? launch_window(g->d.mode, wa, ext, rows, t, at, q & 1, g->dft_pending + at, s)
                             : launch_window64(g->d.mode, g->win64, t, at, q & 1, g->dft_pending + at, s);
     }
     g->launches += launch_steps_advance(g->ctrl, n, s);

@@ -318,6 +318,31 @@ struct alignas(16) WinArgs {
 
 // windows along an axis of n cells, each w cells wide, o of them its own
 // (the first and the last own their cells up to the axis' end)
+// What the windows of a grid with poles or TFSF planes take besides.
+struct WinPlane {
+  int axis, lo[2], hi[2];
+  long long off;  // the plane's first cell in the table
+};
+struct WinExt {
+  // poles: P and J of the E components, two copies: J then P of the first pole,
+  // of the second, per component (a grid of Drude poles alone has no P)
+  int np, per;
+  float* pj[2][8];
+  const unsigned short* disp;  // per cell: its material's poles (two bits), its material; 0 without poles
+  const MatF32* mats;
+  // TFSF: the corrections of a stretch of steps, [step][half][cell of the planes]
+  int nplanes;
+  WinPlane plane[kMaxPlanes];
+  const float* tfsf;
+  long long tfsf_cells;
+};
+
+// The FP32 pole updates, one rounding order for the sweeps and the windows
+__device__ __forceinline__ float drude_current(float a, float j, float b, float e) { return __fmaf_rn(a, j, __fmul_rn(b, e)); }
+__device__ __forceinline__ float lorentz_current(float a, float j, float b, float e, float c, float p) {
+  return __fmaf_rn(-c, p, drude_current(a, j, b, e));
+}
+
 __host__ __device__ inline int window_tiles(int n, int w, int o) { return n <= w ? 1 : 1 + (n - w + o - 1) / o; }
 // windows of `rows` rows of an nx x ny grid taking T steps
 inline int window_count(int nx, int ny, int rows, int T) {
@@ -325,7 +350,12 @@ inline int window_count(int nx, int ny, int rows, int T) {
 }
 // T steps from copy `from` of the state to the other, s steps past the
 // counter; DFT samples go to ring slots slot .. slot + T - 1
-int launch_window(int mode, const WinArgs& a, int rows, int T, int s, int from, int slot, cudaStream_t st);
+// (x: null, or what the grid's poles and TFSF planes need)
+int launch_window(int mode, const WinArgs& a, const WinExt* x, int rows, int T, int s, int from, int slot, cudaStream_t st);
+// the materials with poles of every cell
+int launch_window_cells(const FusedArgs& a, unsigned short* disp, cudaStream_t s);
+// the corrections of every TFSF plane cell for nsteps steps from the counter on
+int launch_tfsf_fused_table(int mode, const FusedArgs& a, int nsteps, long long cells, float* out, cudaStream_t s);
 // the same for the windows `items` ((grid << 24) | tile) of a batch
 int launch_window_batch(int mode, const WinArgs* grids, const unsigned* items, int nitems, int T, int s, int from,
                         cudaStream_t st);

@@ -158,23 +158,23 @@ __global__ void __launch_bounds__(256) fused_e_kernel(const __grid_constant__ Fu
         for (int q = 0; q < (MAXP < 0 ? 1 : MAXP); q++) {
           if (q < np) {
             jt[q] = a.J[q][I][c];
-            jsum += jt[q];
+            jsum = __fadd_rn(jsum, jt[q]);
           }
         }
-        e = e + ie * (d[I] - jsum);
+        e = __fmaf_rn(ie, __fsub_rn(d[I], jsum), e);
 #pragma unroll
         for (int q = 0; q < (MAXP < 0 ? 1 : MAXP); q++) {
           if (q >= np) continue;
           if (m.npoles < 0) {
-            a.J[q][I][c] = m.a[q] * jt[q] + m.b[q] * e;
+            a.J[q][I][c] = drude_current(m.a[q], jt[q], m.b[q], e);
           } else {
-            const float pn = a.P[q][I][c] + jt[q];
+            const float pn = __fadd_rn(a.P[q][I][c], jt[q]);
             a.P[q][I][c] = pn;
-            a.J[q][I][c] = m.a[q] * jt[q] + m.b[q] * e - m.c[q] * pn;
+            a.J[q][I][c] = lorentz_current(m.a[q], jt[q], m.b[q], e, m.c[q], pn);
           }
         }
       } else {
-        e = e + ie * d[I];
+        e = __fmaf_rn(ie, d[I], e);
       }
       a.E[I][c] = e + (I == 0 ? add0 : (I == 1 ? add1 : add2));
     }

@@ -107,7 +107,7 @@ __device__ __forceinline__ void tfsf_cell(const FusedArgs& a, int ft, int q, con
     for (int I = 0; I < 3; I++) {
       const int K = third(I, pp.axis);
       const bool has = ft == 0 ? hasE(MODE, I) && hasH(MODE, K) : hasH(MODE, I) && hasE(MODE, K);
-      if (I != pp.axis && has) corr[I] += plane_corr<MODE>(a, pp, row, ft, I, idx, inv_dx);
+      if (I != pp.axis && has) corr[I] = __dadd_rn(corr[I], plane_corr<MODE>(a, pp, row, ft, I, idx, inv_dx));
     }
   }
   if (ft == 0) {
@@ -121,7 +121,7 @@ __device__ __forceinline__ void tfsf_cell(const FusedArgs& a, int ft, int q, con
       if (!(comps >> I & 1)) continue;
       const float dE = static_cast<float>(sc * corr[I]);
       a.E[I][c] = f0[I] + dE;
-      for (int pq = 0; pq < np && pq < 2; pq++) a.J[pq][I][c] += m.b[pq] * dE;
+      for (int pq = 0; pq < np && pq < 2; pq++) a.J[pq][I][c] = __fmaf_rn(m.b[pq], dE, a.J[pq][I][c]);
     }
   } else {
     // the correction goes to B; H = B/(mu_r mu0)
@@ -151,6 +151,78 @@ __global__ void __launch_bounds__(128) tfsf_fused_kernel(const __grid_constant__
     idx[p.axis] = w;
     tfsf_cell<MODE>(a, ft, q, idx);
   }
+}
+
+// The corrections of 2D grids for the steps blockIdx.z from the counter on, for
+// the windows (kernels_window.cu): tfsf_cell's value of the one component that a
+// plane corrects, summed over the planes at the first that corrects the cell's
+// component (zero at the others).
+template <int MODE>
+__global__ void __launch_bounds__(128) tfsf_fused_table_kernel(const __grid_constant__ FusedArgs a, long long cells, float* out) {
+  const int q = blockIdx.y;
+  const PlaneDev& p = a.planes[q];
+  const long long ex = p.hi[0] - p.lo[0] + 1, n = ex * (p.hi[1] - p.lo[1] + 1);
+  const long long at = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (at >= n || p.axis > 1) return;
+  const int i = p.lo[0] + static_cast<int>(at % ex), j = p.lo[1] + static_cast<int>(at / ex);
+  const int idx[3] = {i, j, 0};
+  const long long c = static_cast<long long>(j) * a.pitch + i;
+  int mid = 0;
+  if (a.ids) mid = a.ids[c];
+  else if (a.bids) mid = a.bids[(j >> a.bshift) * a.nbx + (i >> a.bshift)];
+  const MatF32& m = a.mats[mid];
+  const float iemap = a.inv_eps_map ? a.inv_eps_map[c] : 0.f;
+  const double inv_dx = 1.0 / a.dx;
+  const int s = blockIdx.z;
+  const long long t = a.ctrl->t + s;
+#pragma unroll
+  for (int ft = 0; ft < 2; ft++) {
+    const long long row = t - a.ctrl->t0 + (ft == 0 ? 0 : 1);
+    double corr = 0.0;
+    bool first = true;
+    int I = -1;
+#pragma unroll
+    for (int X = 0; X < 3; X++)
+#pragma unroll
+      for (int A = 0; A < 2; A++)
+        if (X != A && A == p.axis && (ft == 0 ? hasE(MODE, X) && hasH(MODE, third(X, A)) : hasH(MODE, X) && hasE(MODE, third(X, A)))) I = X;
+    for (int q1 = 0; q1 < a.nplanes; q1++) {
+      const PlaneDev& pp = a.planes[q1];
+      if (!in_plane(pp, i, j, 0)) continue;
+#pragma unroll
+      for (int X = 0; X < 3; X++) {
+        const int K = third(X, pp.axis);
+        const bool has = ft == 0 ? hasE(MODE, X) && hasH(MODE, K) : hasH(MODE, X) && hasE(MODE, K);
+        if (X != I || X == pp.axis || !has) continue;
+        if (q1 < q) first = false;
+        corr = __dadd_rn(corr, plane_corr<MODE>(a, pp, row, ft, X, idx, inv_dx));
+      }
+    }
+    float v;
+    if (ft == 0) {
+      float ie = m.inv_eps;
+      if (m.npoles == 0 && iemap > 0.f) ie = iemap;
+      const double sc = a.dt / kEps0 * ie;
+      v = static_cast<float>(sc * corr);
+    } else {
+      const double sc = a.eta * a.dt / kMu0 * (a.has_mu ? static_cast<double>(m.inv_mu) : 1.0);
+      v = -static_cast<float>(sc * corr);
+    }
+    out[(static_cast<long long>(s) * 2 + ft) * cells + p.off + at] = first ? v : 0.f;
+  }
+}
+
+int launch_tfsf_fused_table(int mode, const FusedArgs& a, int nsteps, long long cells, float* out, cudaStream_t s) {
+  if (a.nplanes == 0) return 0;
+  long long most = 1;
+  for (int q = 0; q < a.nplanes; q++) {
+    const PlaneDev& p = a.planes[q];
+    most = std::max(most, static_cast<long long>(p.hi[0] - p.lo[0] + 1) * (p.hi[1] - p.lo[1] + 1));
+  }
+  const dim3 grid(static_cast<unsigned>((most + 127) / 128), a.nplanes, nsteps);
+  if (mode == kTE) tfsf_fused_table_kernel<kTE><<<grid, 128, 0, s>>>(a, cells, out);
+  else tfsf_fused_table_kernel<kTM><<<grid, 128, 0, s>>>(a, cells, out);
+  return 1;
 }
 
 int launch_tfsf_fused(int mode, const FusedArgs& a, int ft, cudaStream_t s) {

@@ -193,6 +193,78 @@ __device__ __forceinline__ void sample_regions(const Region* reg, unsigned set, 
   }
 }
 
+// Grids with poles or TFSF planes (EXT, kernels of their own, so that the others
+// keep their registers). What bounded them was, as for the rest, the chain of
+// launches: 9.9 us a step at 160 x 96 TE with Drude cells, 18.3 with TFSF planes
+// too, now 2.3 and 4.7; 3000 x 2000 78, 88 and (a Lorentz pole in most cells)
+// 140 us, now 22, 35 and 108. J, P and the poles' coefficients of every cell lie
+// in shared memory, where the rows of a warp that hold poles take them as packed
+// pairs (looked up per cell through the material table, a Lorentz pole's 3000 x
+// 2000 took 168 us: slower than the launches per half step). The corrections of
+// the planes come from a table of the stretch's steps, formed by one launch
+// ahead of its windows: they need only the auxiliary grids.
+struct PlaneAct {
+  int comp, lo[2], hi[2], ex;
+  const float* at;  // value of window cell (0, 0) at the launch's first step
+};
+struct ExtShared {
+  PlaneAct plane[2][kMaxPlanes];
+  int nplane[2];
+};
+
+// one warp: lane 2 q + half
+__device__ __forceinline__ void list_planes(const WinExt& x, ExtShared& es, int mode, int x0, int y0, int rows, int s, int lane) {
+  const int q = lane >> 1, h = lane & 1;
+  PlaneAct t{};
+  bool in = false;
+  if (q < x.nplanes) {
+    const WinPlane& p = x.plane[q];
+    const bool te = mode == kTE;
+    // the component that a plane of this normal corrects
+    if (h == 0) t.comp = te ? 1 - p.axis : 2;
+    else t.comp = te ? 2 : 1 - p.axis;
+    for (int d = 0; d < 2; d++) {
+      t.lo[d] = max(p.lo[d] - (d ? y0 : x0), 0);
+      t.hi[d] = min(p.hi[d] - (d ? y0 : x0), (d ? rows : kWinCols) - 1);
+    }
+    t.ex = p.hi[0] - p.lo[0] + 1;
+    t.at = x.tfsf + (static_cast<long long>(s) * 2 + h) * x.tfsf_cells + p.off + static_cast<long long>(y0 - p.lo[1]) * t.ex + (x0 - p.lo[0]);
+    in = p.axis < 2 && t.lo[0] <= t.hi[0] && t.lo[1] <= t.hi[1];
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const unsigned set = __ballot_sync(kAll, in && h == k);
+    if (in && h == k) es.plane[k][__popc(set & ((1u << lane) - 1))] = t;
+    if (lane == 0) es.nplane[k] = __popc(set);
+  }
+}
+
+// a cell's entry in WinExt::disp: its poles, its material
+__device__ __forceinline__ int poles_of(unsigned mid) { return mid >> 14; }
+__device__ __forceinline__ const MatF32& material_of(const WinExt& x, unsigned mid) { return x.mats[mid & 0x3fffu]; }
+
+// a correction v of E moves every pole's current by b * v
+__device__ __noinline__ void kick_poles(const WinExt& x, float* at, int n, unsigned mids, pair_t v) {
+  const float2 d = unpack(v);
+#pragma unroll 1
+  for (int c = 0; c < 2; c++) {
+    const unsigned mid = c ? mids >> 16 : mids & 0xffffu;
+    const int np = poles_of(mid);
+    for (int q = 0; q < np; q++) {
+      float* j = at + c + q * x.per * n;
+      *j = __fmaf_rn(material_of(x, mid).b[q], c ? d.y : d.x, *j);
+    }
+  }
+}
+
+struct NoExt {};
+
+// arrays of the window's cells in shared memory: the integrators, J and P, the
+// coefficients
+__host__ __device__ __forceinline__ int ext_arrays(int mode, const WinExt& x) {
+  return 4 + (mode == kTE ? 2 : 1) * x.np * x.per + x.np * (1 + x.per);
+}
+
 }  // namespace
 
 struct WinSpan {
@@ -203,11 +275,13 @@ struct WinSpan {
 // One window, T steps. GEN: the window touches the outer ring, the CPML, a
 // source or a DFT region; otherwise every cell is interior with the plain
 // coefficients and nothing else acts on it.
-template <int MODE, bool XFIRST, bool GEN, bool CAP, int NW, int R>
-__device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, float* psi, const WinSpan& sp, int T,
+template <int MODE, bool XFIRST, bool GEN, bool CAP, int NW, int R, class Ext>
+__device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] const Ext& x, [[maybe_unused]] const ExtShared* es,
+                                           Shared<NW, R>& sh, float* psi, const WinSpan& sp, int T,
                                            int from, int slot, long long t0, pair_t (&f0)[R], pair_t (&f1)[R], pair_t (&f2)[R],
                                            pair_t (&ie)[R]) {
   constexpr bool TE = MODE == kTE;
+  constexpr bool EXT = GEN && std::is_same<Ext, WinExt>::value;
   constexpr int N = kWinCols * Shared<NW, R>::kRows;  // cells of the window: one integrator array
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = w * R, c0 = sp.x0 + 2 * lane, j0 = sp.y0 + row0;
@@ -266,6 +340,105 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
     for (int k = 0; k < sh.nreg[1]; k++)
       if (sh.reg[1][k].hi[1] >= row0 && sh.reg[1][k].lo[1] < row0 + R) reg_h |= 1u << k;
   }
+  // EXT: the warp's rows with poles, its planes; J and P follow the integrators,
+  // then the poles' coefficients a, b (and c) in every cell, zero without poles
+  unsigned rows_p = 0, mine_p[2] = {0, 0};
+  int npj = 0, per_comp = 0;  // arrays of a component
+  const unsigned* mids = nullptr;
+  float* const pj_at = psi_at + 4 * N;
+  [[maybe_unused]] float* co_at = nullptr;
+  if constexpr (EXT) {
+    per_comp = x.np * x.per;
+    npj = (TE ? 2 : 1) * per_comp;
+    const int nco = (1 + x.per) * x.np;
+    co_at = pj_at + npj * N;
+    unsigned* const mid_at = reinterpret_cast<unsigned*>(psi + (4 + npj + nco) * N) + row0 * 32 + lane;
+    mids = mid_at;
+    if (x.np > 0) {
+#pragma unroll 1
+      for (int r = 0; r < R; r++) {
+        unsigned m = mid_at[r * 32];  // both cells; none of the ring
+        if (!(rows_in >> r & 1)) m = 0;
+        if (!ok0) m &= 0xffff0000u;
+        if (!ok1) m &= 0xffffu;
+        mid_at[r * 32] = m;
+        if (!__any_sync(kAll, m != 0)) continue;
+        rows_p |= 1u << r;
+        const int n0 = poles_of(m & 0xffffu), n1 = poles_of(m >> 16);
+        for (int k = 0; k < npj; k++) {
+          const int q = k % per_comp / x.per;
+          float2 v = make_float2(0.f, 0.f);
+          if (m) v = unpack(load_l2(x.pj[from][k] + static_cast<long long>(j0 + r) * pitch + c0));
+          store_pair(pj_at + r * kWinCols + k * N, pack(q < n0 ? v.x : 0.f, q < n1 ? v.y : 0.f));
+        }
+        for (int q = 0; q < x.np; q++) {
+          const MatF32* const m0 = q < n0 ? &material_of(x, m) : nullptr;
+          const MatF32* const m1 = q < n1 ? &material_of(x, m >> 16) : nullptr;
+          float* co = co_at + r * kWinCols + q * (1 + x.per) * N;
+          store_pair(co, pack(m0 ? m0->a[q] : 0.f, m1 ? m1->a[q] : 0.f));
+          store_pair(co + N, pack(m0 ? m0->b[q] : 0.f, m1 ? m1->b[q] : 0.f));
+          if (x.per == 2) store_pair(co + 2 * N, pack(m0 ? -m0->c[q] : 0.f, m1 ? -m1->c[q] : 0.f));
+        }
+      }
+    }
+    for (int h = 0; h < 2; h++)
+      for (int k = 0; k < es->nplane[h]; k++)
+        if (es->plane[h][k].hi[1] >= row0 && es->plane[h][k].lo[1] < row0 + R) mine_p[h] |= 1u << k;
+  }
+  // sum of the currents of component q's poles in row r, and their update
+  auto currents = [&](int q, int r) {
+    pair_t s = 0;
+    if constexpr (EXT) {
+      const float* p = pj_at + q * per_comp * N + r * kWinCols;
+      s = load_pair(p);
+      if (x.np > 1) s = add2(s, load_pair(p + x.per * N));
+    }
+    return s;
+  };
+  // drude_current and lorentz_current (a Drude pole's c is zero; its P is not
+  // written back); a cell without the pole keeps its zero whatever E is
+  auto advance = [&](int comp, int r, pair_t e) {
+    if constexpr (EXT) {
+#pragma unroll 1
+      for (int q = 0; q < x.np; q++) {
+        float* const j = pj_at + (comp * per_comp + q * x.per) * N + r * kWinCols;
+        const float* const co = co_at + q * (1 + x.per) * N + r * kWinCols;
+        const pair_t jt = load_pair(j);
+        pair_t v = fma2(load_pair(co), jt, mul2(load_pair(co + N), e));
+        if (x.per == 2) {
+          const pair_t pn = add2(load_pair(j + N), jt);
+          store_pair(j + N, pn);
+          v = fma2(load_pair(co + 2 * N), pn, v);
+        }
+        const float2 now = unpack(v);
+        const unsigned m = mids[r * 32];
+        store_pair(j, pack(q < poles_of(m & 0xffffu) ? now.x : 0.f, q < poles_of(m >> 16) ? now.y : 0.f));
+      }
+    }
+  };
+  // the planes' corrections of half h; fa and fb the (one or) two components
+  auto planes = [&](int h, int st, pair_t (&fa)[R], int ca, pair_t (&fb)[R]) {
+    if constexpr (EXT) {
+#pragma unroll 1
+      for (unsigned m = mine_p[h]; m; m &= m - 1) {
+        const PlaneAct& t = es->plane[h][__ffs(m) - 1];
+        const Cols c(2 * lane, t.lo[0], t.hi[0]);
+        const int lo = t.lo[1] - row0, hi = t.hi[1] - row0;
+        const bool first = t.comp == ca;
+        const float* p = t.at + st * 2 * x.tfsf_cells + static_cast<long long>(row0) * t.ex + 2 * lane;
+        if (!__any_sync(kAll, c.k0 || c.k1)) continue;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r < lo || r > hi) continue;
+          const pair_t v = pack(c.k0 ? __ldcg(p + static_cast<long long>(r) * t.ex) : 0.f,
+                                c.k1 ? __ldcg(p + static_cast<long long>(r) * t.ex + 1) : 0.f);
+          if (first) fa[r] = add2(fa[r], v);
+          else fb[r] = add2(fb[r], v);
+          if (h == 0 && (rows_p >> r & 1)) kick_poles(x, pj_at + (first ? 0 : 1) * per_comp * N + r * kWinCols, N, mids[r * 32], v);
+        }
+      }
+    }
+  };
   // which terms the warp's update has, alike for its lanes: x slab, y slab,
   // flux sources (the update is instantiated for each, free of branches)
   const bool has_x = GEN && __any_sync(kAll, xs >= 0), has_y = GEN && rows_y != 0;
@@ -297,7 +470,7 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
   };
   // One half step of the rows r0 .. r1 - 1. X, Y: the curl terms gain psi*G
   // and psi becomes B*psi + C*raw, the x slab by columns, the y slab by rows
-  auto e_rows = [&](auto X, auto Y, auto FL, int r0, int r1, pair_t below0, int st) {
+  auto e_rows = [&](auto X, auto Y, auto FL, auto PO, int r0, int r1, pair_t below0, int st) {
     const pair_t fx = GEN ? sh.xp[0][0][lane] : fxc[0];
     pair_t bx = 0, cx = 0, gx = 0;
     if (X.value) {
@@ -332,8 +505,17 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
           flux(0, 0, r, st, dx);
           flux(0, 1, r, st, dy);
         }
+        const bool poles = PO.value && (rows_p >> r & 1);
+        if (poles) {
+          dx = sub2(dx, currents(0, r));
+          dy = sub2(dy, currents(1, r));
+        }
         f0[r] = fma2(ie[r], dx, f0[r]);
         f1[r] = fma2(ie[r], dy, f1[r]);
+        if (poles) {
+          advance(0, r, f0[r]);
+          advance(1, r, f1[r]);
+        }
       } else {
         const pair_t rzx = sub2(f2[r], left), rzy = sub2(below, f1[r]);
         pair_t dz = dot2(fx, rzx, fy, rzy);
@@ -355,7 +537,10 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
         }
         if (X.value && !XFIRST) xterm();
         if (FL.value) flux(0, 2, r, st, dz);
+        const bool poles = PO.value && (rows_p >> r & 1);
+        if (poles) dz = sub2(dz, currents(0, r));
         f0[r] = fma2(ie[r], dz, f0[r]);
+        if (poles) advance(0, r, f0[r]);
       }
     }
   };
@@ -422,7 +607,9 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
   };
   using Yes = std::true_type;
   using No = std::false_type;
-  auto e_half = [&](auto X, auto Y, auto FL, int st) { e_rows(X, Y, FL, 0, R, sh.edge_h[w][lane], st); };
+  auto e_half = [&](auto X, auto Y, auto FL, int st) { e_rows(X, Y, FL, No(), 0, R, sh.edge_h[w][lane], st); };
+  // warps with poles: with and without the other terms
+  auto e_half_poles = [&](auto all, int st) { e_rows(all, all, all, Yes(), 0, R, sh.edge_h[w][lane], st); };
   auto h_half = [&](auto X, auto Y, auto FL, int st) { h_rows(X, Y, FL, 0, R, sh.edge_e[w + 1][lane], st); };
 
 #pragma unroll 1
@@ -430,16 +617,26 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
     // ---- E half
     if (GEN && __builtin_expect(mine != 0, 0))
       apply_entries(sh.entry, mine & (sh.kinds[0][0] | sh.kinds[0][1]), sh.undo, st, row0, lane, f0, TE ? 0 : 2, f1);
-    if constexpr (!GEN) e_half(No(), No(), No(), st);
+    bool done = false;
+    if constexpr (EXT) {
+      if (rows_p) {
+        done = true;
+        if (has_x || has_y || has_flux) e_half_poles(Yes(), st);
+        else e_half_poles(No(), st);
+      }
+    }
+    if (EXT && done) {
+    } else if constexpr (!GEN) e_half(No(), No(), No(), st);
     else if (__builtin_expect(has_flux, 0)) e_half(Yes(), Yes(), Yes(), st);
     else if (has_x && has_y) e_half(Yes(), Yes(), No(), st);
     else if (has_x) e_half(Yes(), No(), No(), st);
     else if (has_y) e_half(No(), Yes(), No(), st);
     else e_half(No(), No(), No(), st);
-    if (GEN && __builtin_expect(mine != 0, 0)) {
+    if (GEN && __builtin_expect(mine != 0, 0))
       apply_entries(sh.entry, mine & sh.kinds[0][1], sh.put, st, row0, lane, f0, TE ? 0 : 2, f1);
+    if (EXT && __builtin_expect(mine_p[0] != 0, 0)) planes(0, st, f0, TE ? 0 : 2, f1);
+    if (GEN && __builtin_expect(mine != 0, 0))
       apply_entries(sh.entry, mine & sh.kinds[0][0], sh.put, st, row0, lane, f0, TE ? 0 : 2, f1);
-    }
     sh.edge_e[w][lane] = f0[0];
     if (GEN && __builtin_expect(reg_e != 0, 0))
       sample_regions(sh.reg[0], reg_e, (slot + st) * a.dft_pts[0], row0, lane, f0, TE ? 0 : 2, f1);
@@ -457,10 +654,14 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
     else if (has_x) h_half(Yes(), No(), No(), st);
     else if (has_y) h_half(No(), Yes(), No(), st);
     else h_half(No(), No(), No(), st);
-    if (GEN && __builtin_expect(mine != 0, 0)) {
+    if (GEN && __builtin_expect((EXT ? mine | mine_p[1] : mine) != 0, 0)) {
       for (int kind = 1; kind >= 0; kind--) {
         if (TE) apply_entries(sh.entry, mine & sh.kinds[1][kind], sh.put, st, row0, lane, f2, 2, f2);
         else apply_entries(sh.entry, mine & sh.kinds[1][kind], sh.put, st, row0, lane, f1, 0, f2);
+        if (EXT && kind == 1 && mine_p[1]) {
+          if (TE) planes(1, st, f2, 2, f2);
+          else planes(1, st, f1, 0, f2);
+        }
       }
     }
     sh.edge_h[w + 1][lane] = TE ? f2[R - 1] : f1[R - 1];
@@ -507,15 +708,31 @@ __device__ __forceinline__ void window_run(const WinArgs& a, Shared<NW, R>& sh, 
       put(a.psi[from][1], a.psi[to][1], p, load_pair(psi_at + r * kWinCols + N), true);
       put(a.psi[from][3], a.psi[to][3], p, load_pair(psi_at + r * kWinCols + 3 * N), true);
     }
+    if constexpr (EXT) {
+      if (!(rows_p >> r & 1)) continue;
+      const unsigned m = mids[r * 32];
+      const long long p = j * pitch + c0;
+#pragma unroll 1
+      for (int c = 0; c < 2; c++) {
+        const unsigned mid = c ? m >> 16 : m & 0xffffu;
+        if (!mid) continue;
+        const int n = material_of(x, mid).npoles;
+        for (int k = 0; k < npj; k++) {
+          const int kk = k % per_comp;
+          if (kk / x.per < (n < 0 ? 1 : n) && !(n < 0 && kk % x.per)) x.pj[to][k][p + c] = pj_at[r * kWinCols + k * N + c];
+        }
+      }
+    }
   }
 }
 
 // The window of tile `tile` of a grid: first cell, owned cells, what acts in
 // it; then the steps.
-template <int MODE, bool XFIRST, bool CAP, int NW, int R>
-__device__ __forceinline__ void window_tile(const WinArgs& a, Shared<NW, R>& sh, float* psi, int tile, int T, int s, int from,
+template <int MODE, bool XFIRST, bool CAP, int NW, int R, class Ext>
+__device__ __forceinline__ void window_tile(const WinArgs& a, const Ext& x, ExtShared* es, Shared<NW, R>& sh, float* psi, int tile, int T, int s, int from,
                                             int slot) {
   constexpr int rows = Shared<NW, R>::kRows;
+  constexpr bool EXT = std::is_same<Ext, WinExt>::value;
   const int hx = (T + 1) & ~1;  // columns of a lane come in pairs: an even halo keeps them aligned
   const int ow = kWinCols - 2 * hx, oh = rows - 2 * T;
   const int tiles_x = window_tiles(a.nx, kWinCols, ow);
@@ -578,6 +795,8 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, Shared<NW, R>& sh,
     const unsigned set = __ballot_sync(kAll, in);
     if (in) sh.reg[h][__popc(set & ((1u << lane) - 1))] = o;
     if (lane == 0) sh.nreg[h] = __popc(set);
+  } else if (tid >= 192 && tid < 224) {
+    if constexpr (EXT) list_planes(x, *es, MODE, sp.x0, sp.y0, rows, s, tid & 31);
   }
   // TE: Ex, Ey, Hz; TM: Ez, Hx, Hy
   pair_t f0[R], f1[R], f2[R], ie[R];
@@ -587,6 +806,19 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, Shared<NW, R>& sh,
     const bool in = c0 < a.nx && j0 + r < a.ny;
     ie[r] = both(a.ie0);
     if (a.ie) ie[r] = in ? load_pair(a.ie + (j0 + r) * static_cast<long long>(a.pitch) + c0) : 0ull;
+  }
+  bool poles = false;
+  if constexpr (EXT) {
+    if (x.np > 0) {
+      unsigned* const mids = reinterpret_cast<unsigned*>(psi + ext_arrays(MODE, x) * kWinCols * rows);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const bool in = c0 < a.nx && j0 + r < a.ny;
+        const unsigned m = in ? *reinterpret_cast<const unsigned*>(x.disp + (j0 + r) * static_cast<long long>(a.pitch) + c0) : 0u;
+        mids[((tid >> 5) * R + r) * 32 + (tid & 31)] = m;
+        poles = poles || m != 0;
+      }
+    }
   }
   after_previous_launch();
   const long long t0 = a.ctrl->t + s;
@@ -598,12 +830,14 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, Shared<NW, R>& sh,
     f1[r] = in ? load_l2(a.f[from][1] + c) : 0ull;
     f2[r] = in ? load_l2(a.f[from][2] + c) : 0ull;
   }
-  __syncthreads();
+  if (EXT) poles = __syncthreads_or(poles);
+  else __syncthreads();
   entry_values<NW, R>(a, sh, T, t0, from);
-  const bool plain = sp.x0 >= a.plain[0][0] && sp.x0 + kWinCols - 1 <= a.plain[0][1] && sp.y0 >= a.plain[1][0] &&
+  bool plain = sp.x0 >= a.plain[0][0] && sp.x0 + kWinCols - 1 <= a.plain[0][1] && sp.y0 >= a.plain[1][0] &&
                      sp.y0 + rows - 1 <= a.plain[1][1] && sh.nentry + sh.nreg[0] + sh.nreg[1] == 0;
-  if (plain) window_run<MODE, XFIRST, false, CAP, NW, R>(a, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
-  else window_run<MODE, XFIRST, true, CAP, NW, R>(a, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
+  if constexpr (EXT) plain = plain && !poles && es->nplane[0] + es->nplane[1] == 0;
+  if (plain) window_run<MODE, XFIRST, false, CAP, NW, R>(a, x, es, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
+  else window_run<MODE, XFIRST, true, CAP, NW, R>(a, x, es, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
   // the soft sources' last values, by the window that owns the source cell
   if (tid < a.nsrc) {
     const SourceDev& q = a.src[tid];
@@ -618,7 +852,17 @@ __global__ void __launch_bounds__(32 * NW, 2) window_kernel(const __grid_constan
   extern __shared__ __align__(16) float psi[];
   __shared__ Shared<NW, R> sh;
   let_next_launch_start();
-  window_tile<MODE, true, CAP, NW, R>(a, sh, psi, blockIdx.x, T, s, from, slot);
+  window_tile<MODE, true, CAP, NW, R>(a, NoExt{}, nullptr, sh, psi, blockIdx.x, T, s, from, slot);
+}
+
+template <int MODE, int NW, int R>
+__global__ void __launch_bounds__(32 * NW, 2) window_ext_kernel(const __grid_constant__ WinArgs a, const __grid_constant__ WinExt x,
+                                                                int T, int s, int from, int slot) {
+  extern __shared__ __align__(16) float psi[];
+  __shared__ Shared<NW, R> sh;
+  __shared__ ExtShared es;
+  let_next_launch_start();
+  window_tile<MODE, true, false, NW, R>(a, x, &es, sh, psi, blockIdx.x, T, s, from, slot);
 }
 
 // a batch: item = (grid index << 24) | tile; the grid's arguments are copied
@@ -636,7 +880,7 @@ __global__ void __launch_bounds__(32 * NW, 2) window_batch_kernel(const WinArgs*
   for (int q = threadIdx.x; q < static_cast<int>(sizeof(WinArgs) / 16); q += blockDim.x)
     reinterpret_cast<int4*>(raw)[q] = src[q];
   __syncthreads();
-  window_tile<MODE, false, false, NW, R>(*reinterpret_cast<const WinArgs*>(raw), sh, psi, static_cast<int>(w & 0xffffffu), T, s,
+  window_tile<MODE, false, false, NW, R>(*reinterpret_cast<const WinArgs*>(raw), NoExt{}, nullptr, sh, psi, static_cast<int>(w & 0xffffffu), T, s,
                                   from, 0);
 }
 
@@ -653,8 +897,53 @@ void window_go(F fn, int n, cudaStream_t st, A... args) {
 
 }  // namespace
 
-int launch_window(int mode, const WinArgs& a, int rows, int T, int s, int from, int slot, cudaStream_t st) {
+namespace {
+
+__global__ void window_cells_kernel(const __grid_constant__ FusedArgs a, unsigned short* disp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= a.pitch || j >= a.ny) return;
+  const long long c = static_cast<long long>(j) * a.pitch + i;
+  int mid = 0;
+  if (i < a.nx && a.ids) mid = a.ids[c];
+  else if (i < a.nx && a.bids) mid = a.bids[(j >> a.bshift) * a.nbx + (i >> a.bshift)];
+  const int n = i < a.nx ? a.mats[mid].npoles : 0;
+  disp[c] = static_cast<unsigned short>(n == 0 ? 0 : (n < 0 ? 1 : n) << 14 | mid);
+}
+
+size_t ext_bytes(int mode, const WinExt& x, int rows) {
+  const size_t cells = static_cast<size_t>(kWinCols) * rows;
+  return ext_arrays(mode, x) * cells * sizeof(float) + (x.np > 0 ? cells * sizeof(unsigned short) : 0);
+}
+
+template <int NW, int R, typename F>
+void window_ext_go(F fn, int mode, int n, cudaStream_t st, const WinArgs& a, const WinExt& x, int T, int s, int from, int slot) {
+  once_per_device(reinterpret_cast<const void*>(fn), [&] {
+    WinExt most{};
+    // (windows of 64 rows hold one Drude pole at most)
+    most.np = most.per = NW * R == 64 ? 1 : 2;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ext_bytes(mode, most, NW * R)));
+  });
+  launch_chained(fn, dim3(n), dim3(32 * NW), ext_bytes(mode, x, NW * R), st, a, x, T, s, from, slot);
+}
+
+}  // namespace
+
+int launch_window_cells(const FusedArgs& a, unsigned short* disp, cudaStream_t s) {
+  window_cells_kernel<<<dim3((a.pitch + 31) / 32, (a.ny + 7) / 8), dim3(32, 8), 0, s>>>(a, disp);
+  return 1;
+}
+
+int launch_window(int mode, const WinArgs& a, const WinExt* x, int rows, int T, int s, int from, int slot, cudaStream_t st) {
   const int n = window_count(a.nx, a.ny, rows, T);
+  if (x) {
+    auto ext = [&](auto small, auto large) {
+      if (rows == 32) window_ext_go<16, 2>(small, mode, n, st, a, *x, T, s, from, slot);
+      else window_ext_go<16, 4>(large, mode, n, st, a, *x, T, s, from, slot);
+    };
+    if (mode == kTE) ext(window_ext_kernel<kTE, 16, 2>, window_ext_kernel<kTE, 16, 4>);
+    else ext(window_ext_kernel<kTM, 16, 2>, window_ext_kernel<kTM, 16, 4>);
+    return 1;
+  }
   auto go = [&](auto small, auto large) {
     if (rows == 32) window_go<16, 2>(small, n, st, a, T, s, from, slot);
     else window_go<16, 4>(large, n, st, a, T, s, from, slot);

@@ -156,3 +156,41 @@ def test_fp64_windows_with_divisors_at_the_ends_of_the_range(fdtd, mode, eps, mu
         assert np.array_equal(a, b, equal_nan=True)
         ok = ~np.isnan(a)
         assert np.array_equal(np.signbit(a[ok]), np.signbit(b[ok]))
+
+
+@pytest.mark.parametrize("mode", [P.TE, P.TM], ids=["te", "tm"])
+@pytest.mark.parametrize("nx,ny,poles", [(3, 3, 1), (31, 64, 0), (64, 32, -1), (65, 33, 1), (113, 47, 2), (112, 48, 0),
+                                         (130, 66, -1), (200, 131, 2), (410, 300, 1), (701, 590, -1)])
+def test_windows_with_poles_and_planes(fdtd, mode, nx, ny, poles):
+    """FP32 windows of grids with poles (-1: Drude alone, which keeps no P) and
+    TFSF planes: each window's edges, cells of every material in one row, pole
+    cells on planes, on box edges and under sources; a grid of one material with
+    poles; J and P left in cells whose material has none are not touched."""
+    p = _problem64(mode, nx, ny, nx + ny, abs(poles))
+    dt = p.dt
+    if poles == -1:
+        p.materials[2] = P.Material.drude(2.0, 0.15 / dt, 0.03 / dt)
+    if (nx, ny) == (65, 33):
+        p.materials, p.ids, p.eps_map = p.materials[2:], None, None
+    E, H, _, _ = mode_fields(mode)
+    names = E + H + ["Px", "Py", "Pz", "Jx", "Jy", "Jz"] + list(fdtd.PSI_NAMES)
+    rng = np.random.default_rng(3)
+    stray = rng.normal(size=(1, ny, nx)) * 1e-3
+    out = []
+    for kind in ("auto", "regs"):
+        g = fdtd.Grid.from_problem(p, "f32")
+        g.set_sweep_kernel(kind)
+        if poles:
+            g.set("J" + E[0][1], stray)
+        for n in (1, 2, 3, 13, 64, 71):
+            g.step(n)
+        vals = []
+        for n in names:
+            try:
+                vals.append(g.get(n))
+            except fdtd.FdtdError:
+                pass
+        out.append(vals + [g.dft(h) for h in g.dft_handles])
+    assert any(np.any(v) for v in out[0])
+    for q, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a, b), (q, float(np.abs(a - b).max()))
