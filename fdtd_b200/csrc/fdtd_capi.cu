@@ -132,7 +132,7 @@ struct BoxSourceH {
 struct AuxH {
   int ncells, L;
   std::vector<double> vals;
-  double *d_state = nullptr;  // Dz, Ez, By, Hy, psiE, psiH (6L)
+  double *d_state = nullptr;  // Dz, Ez, By, Hy, psiE, psiH (6L), and a second copy of them
   double *d_coef = nullptr;   // 8L
   double *d_vals = nullptr;
   double *d_tab = nullptr;    // 2 * cap * L
@@ -545,7 +545,7 @@ int build_aux(fdtd_grid* g, AuxH& a) {
   }
   int rc = upload_vec(g, reinterpret_cast<void**>(&a.d_coef), coef.data(), coef.size() * sizeof(double));
   if (rc) return rc;
-  rc = dalloc(g, reinterpret_cast<void**>(&a.d_state), 6 * static_cast<size_t>(L) * sizeof(double));
+  rc = dalloc(g, reinterpret_cast<void**>(&a.d_state), 12 * static_cast<size_t>(L) * sizeof(double));
   if (rc) return rc;
   return upload_vec(g, reinterpret_cast<void**>(&a.d_vals), a.vals.data(),
                     std::max<size_t>(1, a.vals.size()) * sizeof(double));
@@ -1999,8 +1999,7 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
   for (auto& a : g->auxes) {
     double* st = a.d_state;
     const int L = a.L;
-    g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, st + L, st + 2 * L, st + 3 * L, st + 4 * L,
-                                         st + 5 * L, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t,
+    g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t,
                                          nsteps, a.d_tab, a.d_tab + a.cap * L, s);
   }
   // the tables' first row is this step (set on the stream: no host wait)
@@ -2080,8 +2079,7 @@ static int half_step_impl(fdtd_grid* g, int phase, int part, void* stream) {
       }
       double* st = a.d_state;
       const int L = a.L;
-      g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, st + L, st + 2 * L, st + 3 * L, st + 4 * L,
-                                           st + 5 * L, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t, 1,
+      g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t, 1,
                                            a.d_tab, a.d_tab + a.cap * L, s);
     }
     if (!g->auxes.empty()) g->launches += launch_chunk_start(g->ctrl, s);
@@ -3209,8 +3207,7 @@ extern "C" int fdtd_step_static_scratch(fdtd_grid* g, int nsteps, void* stream) 
     p += 2 * static_cast<size_t>(a.cap) * a.L;
     double* st = a.d_state;
     const int L = a.L;
-    g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, st + L, st + 2 * L, st + 3 * L, st + 4 * L,
-                                         st + 5 * L, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t,
+    g->launches += launch_aux_precompute(L, g->d.dt, g->d.dx, st, a.d_coef, a.d_vals, static_cast<int>(a.vals.size()), g->t,
                                          nsteps, a.d_tab, a.d_tab + a.cap * L, s);
   }
   if (naux > 0) {

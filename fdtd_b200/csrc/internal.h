@@ -475,8 +475,7 @@ int launch_staged_eh(const FusedArgs& a, const EhSched& s, int blocks, cudaStrea
 int launch_tfsf_fused(int mode, const FusedArgs& a, int ft, cudaStream_t s);
 int launch_fused3d_e(const FusedArgs& a, cudaStream_t s);
 int launch_fused3d_h(const FusedArgs& a, cudaStream_t s);
-int launch_aux_precompute(int L, double dt, double dx, double* Dz, double* Ez, double* By, double* Hy,
-                          double* psiE, double* psiH, const double* coef, const double* vals, int nvals,
+int launch_aux_precompute(int L, double dt, double dx, double* state, const double* coef, const double* vals, int nvals,
                           long long s0, int nsteps, double* Etab, double* Htab, cudaStream_t s);
 int launch_dft_gather(int precision, const DftRegionDev* regions, int nreg, long long total_pts, long long max_pts,
                       const void* const* fields, int ny, int pitch, int slot, void* buf, cudaStream_t s);

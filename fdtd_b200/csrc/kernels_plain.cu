@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "plain_tfsf.cuh"
+#include "quotient.cuh"
 
 namespace fdtdb {
 
@@ -900,33 +901,25 @@ int launch_material_explicit(int mode, const PlainArgs& a, int ft, cudaStream_t 
 // The chain of steps runs ahead of the main grid's first step, so its latency
 // counts in full: with the state and coefficients read from memory in every
 // pass, a step took 2.4 us at L = 650. Here a thread keeps the state and
-// coefficients of its C cells in registers, Ez and Hy alone pass through shared
+// coefficients of its cell in registers, Ez and Hy alone pass through shared
 // memory, and a step has two barriers; the tables are written behind them.
-template <int C>
 __global__ void __launch_bounds__(1024) aux_kernel(int L, double dt, double* Dz, double* Ez, double* By, double* Hy,
                                                    double* psiE, double* psiH, const double* coef, const double* vals,
                                                    int nvals, long long s0, int nsteps, double* Etab, double* Htab) {
   extern __shared__ double aux_sm[];
   double* const E = aux_sm + 1;      // E[-1 .. L], H[-1 .. L]; the ghosts stay zero
   double* const H = E + L + 2;
-  double D[C], B[C], pE[C], pH[C], eB[C], eC[C], eF[C], eG[C], hB[C], hC[C], hF[C], hG[C];
-  if (threadIdx.x == 0) E[-1] = E[L] = H[-1] = H[L] = 0.0;
+  const int x = threadIdx.x;
+  const bool in = x < L;
+  double D = 0.0, B = 0.0, pE = 0.0, pH = 0.0, co[8] = {};
+  if (x == 0) E[-1] = E[L] = H[-1] = H[L] = 0.0;
+  if (in) {
+    D = Dz[x];
+    B = By[x];
+    pE = psiE[x];
+    pH = psiH[x];
 #pragma unroll
-  for (int c = 0; c < C; c++) {
-    const int x = threadIdx.x + c * blockDim.x;
-    if (x >= L) continue;
-    D[c] = Dz[x];
-    B[c] = By[x];
-    pE[c] = psiE[x];
-    pH[c] = psiH[x];
-    eB[c] = coef[x];
-    eC[c] = coef[L + x];
-    eF[c] = coef[2 * L + x];
-    eG[c] = coef[3 * L + x];
-    hB[c] = coef[4 * L + x];
-    hC[c] = coef[5 * L + x];
-    hF[c] = coef[6 * L + x];
-    hG[c] = coef[7 * L + x];
+    for (int q = 0; q < 8; q++) co[q] = coef[q * L + x];
     Etab[x] = E[x] = Ez[x];
     Htab[x] = H[x] = Hy[x];
   }
@@ -935,15 +928,12 @@ __global__ void __launch_bounds__(1024) aux_kernel(int L, double dt, double* Dz,
     const double src = sa >= 1 && sa <= nvals ? vals[sa - 1] : 0.0;
     __syncthreads();
     // YeeUpdate<TEM,Dz>, UpdatePML<TEM,Electric,X>, VacuumUpdate E, the source
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      const int x = threadIdx.x + c * blockDim.x;
-      if (x >= L) continue;
+    if (in) {
       const double diff = H[x] - H[x - 1];
-      double d = D[c] + dt * (eF[c] * diff + 0.0);
-      d += dt * pE[c] * eG[c];
-      pE[c] = eB[c] * pE[c] + eC[c] * diff;
-      D[c] = d;
+      double d = D + dt * (co[2] * diff + 0.0);
+      d += dt * pE * co[3];
+      pE = co[0] * pE + co[1] * diff;
+      D = d;
       double e = d / kEps0;
       if (x == kAuxNpml + 5) e += src;
       E[x] = e;
@@ -951,34 +941,151 @@ __global__ void __launch_bounds__(1024) aux_kernel(int L, double dt, double* Dz,
     }
     __syncthreads();
     // YeeUpdate<TEM,By>, UpdatePML<TEM,Magnetic,X>, VacuumUpdate H
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      const int x = threadIdx.x + c * blockDim.x;
-      if (x >= L) continue;
+    if (in) {
       const double diff = E[x + 1] - E[x];
-      double b = B[c] + -dt * (0.0 + -hF[c] * diff);
-      b += -dt * pH[c] * hG[c];
-      pH[c] = hB[c] * pH[c] + -hC[c] * diff;
-      B[c] = b;
+      double b = B + -dt * (0.0 + -co[6] * diff);
+      b += -dt * pH * co[7];
+      pH = co[4] * pH + -co[5] * diff;
+      B = b;
       const double h = b / kMu0;
       H[x] = h;
       Htab[static_cast<long long>(s) * L + x] = h;
     }
   }
+  if (!in) return;
+  Dz[x] = D;
+  By[x] = B;
+  psiE[x] = pE;
+  psiH[x] = pH;
+  Ez[x] = E[x];
+  Hy[x] = H[x];
+}
+
+// Rows longer than a CTA's threads. By one CTA with the state in memory a step
+// took 7.5 us at L = 6050. The row is cut, as the 2D grids are
+// (kernels_window.cu), into overlapping windows of 128 cells, a warp each, that
+// take up to 32 steps per launch in registers with a shuffle per half step:
+// values within T cells of a window's end inside the row go stale, the others
+// are exact. An even number of launches alternates between the two copies of the
+// state. Its chain of FP64 operations bounds it: 0.5 us a step at any length
+// (which the kernel above undercuts up to its 1024 cells: 0.45 us at L = 400).
+constexpr int kAuxCells = 4, kAuxWin = 32 * kAuxCells, kAuxSteps = 32;
+
+// the quotients of a lane's cells by b, y = 1 / b
+__device__ __forceinline__ void aux_quotients(const double (&a)[kAuxCells], double b, double y, double (&q)[kAuxCells]) {
+  bool easy = true;
 #pragma unroll
-  for (int c = 0; c < C; c++) {
-    const int x = threadIdx.x + c * blockDim.x;
-    if (x >= L) continue;
-    Dz[x] = D[c];
-    By[x] = B[c];
-    psiE[x] = pE[c];
-    psiH[x] = pH[c];
-    Ez[x] = E[x];
-    Hy[x] = H[x];
+  for (int c = 0; c < kAuxCells; c++) {
+    q[c] = quotient_of(a[c], b, y);
+    easy = easy && quotient_in_range(a[c]);
+  }
+  if (__builtin_expect(!easy, 0)) {
+#pragma unroll
+    for (int c = 0; c < kAuxCells; c++) q[c] = plain_quotient(a[c], b);
   }
 }
 
-// The same with the state in memory, for rows longer than the registers hold.
+__global__ void __launch_bounds__(32) aux_window_kernel(int L, double dt, const double* was, double* now, const double* coef,
+                                                        const double* vals, int nvals, long long s0, int T, int row,
+                                                        double* Etab, double* Htab) {
+  constexpr int C = kAuxCells;
+  constexpr unsigned kWarp = 0xffffffffu;
+  let_next_launch_start();
+  const int lane = threadIdx.x, w0 = blockIdx.x * (kAuxWin - 2 * T), x0 = w0 + lane * C;
+  const int lo = blockIdx.x == 0 ? 0 : w0 + T, hi = w0 + kAuxWin >= L ? L : w0 + kAuxWin - T;  // the cells it owns
+  double D[C], E[C], B[C], H[C], pE[C], pH[C], eB[C], eC[C], eF[C], eG[C], hB[C], hC[C], hF[C], hG[C];
+  bool in[C], own[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    const int x = x0 + c;
+    in[c] = x < L;
+    own[c] = x >= lo && x < hi;
+    auto co = [&](int q) { return in[c] ? coef[q * static_cast<long long>(L) + x] : 0.0; };
+    eB[c] = co(0);
+    eC[c] = co(1);
+    eF[c] = co(2);
+    eG[c] = co(3);
+    hB[c] = co(4);
+    hC[c] = co(5);
+    hF[c] = co(6);
+    hG[c] = co(7);
+  }
+  after_previous_launch();
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    auto st = [&](int q) { return in[c] ? __ldcg(was + q * static_cast<long long>(L) + x0 + c) : 0.0; };
+    D[c] = st(0);
+    E[c] = st(1);
+    B[c] = st(2);
+    H[c] = st(3);
+    pE[c] = st(4);
+    pH[c] = st(5);
+    if (row == 0 && own[c]) {
+      Etab[x0 + c] = E[c];
+      Htab[x0 + c] = H[c];
+    }
+  }
+  // the launch's source values, a step per lane
+  const long long sv = s0 + row + 1 + lane;
+  const double mine = sv >= 1 && sv <= nvals ? vals[sv - 1] : 0.0;
+  double* et = Etab + static_cast<long long>(row) * L + x0;
+  double* ht = Htab + static_cast<long long>(row) * L + x0;
+#pragma unroll 1
+  for (int s = 1; s <= T; s++) {
+    const double src = __shfl_sync(kWarp, mine, s - 1);
+    et += L;
+    ht += L;
+    // YeeUpdate<TEM,Dz>, UpdatePML<TEM,Electric,X>, VacuumUpdate E, the source
+    double left = __shfl_up_sync(kWarp, H[C - 1], 1);
+    if (x0 == 0) left = 0.0;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const double diff = H[c] - left;
+      left = H[c];
+      double d = D[c] + dt * (eF[c] * diff + 0.0);
+      d += dt * pE[c] * eG[c];
+      pE[c] = eB[c] * pE[c] + eC[c] * diff;
+      D[c] = d;
+    }
+    aux_quotients(D, kEps0, 1.0 / kEps0, E);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      if (x0 + c == kAuxNpml + 5) E[c] += src;
+      if (!in[c]) E[c] = 0.0;
+      if (own[c]) et[c] = E[c];
+    }
+    // YeeUpdate<TEM,By>, UpdatePML<TEM,Magnetic,X>, VacuumUpdate H
+    double right = __shfl_down_sync(kWarp, E[0], 1);
+    if (lane == 31) right = 0.0;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const double diff = (c + 1 < C ? E[c + 1 < C ? c + 1 : c] : right) - E[c];
+      double b = B[c] + -dt * (0.0 + -hF[c] * diff);
+      b += -dt * pH[c] * hG[c];
+      pH[c] = hB[c] * pH[c] + -hC[c] * diff;
+      B[c] = b;
+    }
+    aux_quotients(B, kMu0, 1.0 / kMu0, H);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      if (!in[c]) H[c] = 0.0;
+      if (own[c]) ht[c] = H[c];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    if (!own[c]) continue;
+    auto st = [&](int q, double v) { now[q * static_cast<long long>(L) + x0 + c] = v; };
+    st(0, D[c]);
+    st(1, E[c]);
+    st(2, B[c]);
+    st(3, H[c]);
+    st(4, pE[c]);
+    st(5, pH[c]);
+  }
+}
+
+// The same by one CTA with the state in memory, for a step or two.
 __global__ void aux_long_kernel(int L, double dt, double* Dz, double* Ez, double* By, double* Hy, double* psiE,
                                 double* psiH, const double* coef, const double* vals, int nvals, long long s0,
                                 int nsteps, double* Etab, double* Htab) {
@@ -1031,19 +1138,29 @@ __global__ void aux_long_kernel(int L, double dt, double* Dz, double* Ez, double
   }
 }
 
-int launch_aux_precompute(int L, double dt, double dx, double* Dz, double* Ez, double* By, double* Hy,
-                          double* psiE, double* psiH, const double* coef, const double* vals, int nvals,
+int launch_aux_precompute(int L, double dt, double dx, double* state, const double* coef, const double* vals, int nvals,
                           long long s0, int nsteps, double* Etab, double* Htab, cudaStream_t s) {
   (void)dx;
-  const size_t smem = 2 * (static_cast<size_t>(L) + 2) * sizeof(double);
-  const int block = std::min(1024, (L + 31) / 32 * 32);
-  if (L <= 1024)
-    aux_kernel<1><<<1, block, smem, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
-  else if (L <= 2048)
-    aux_kernel<2><<<1, 1024, smem, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
-  else
-    aux_long_kernel<<<1, 1024, 0, s>>>(L, dt, Dz, Ez, By, Hy, psiE, psiH, coef, vals, nvals, s0, nsteps, Etab, Htab);
-  return 1;
+  if (L <= 1024) {
+    const size_t smem = 2 * (static_cast<size_t>(L) + 2) * sizeof(double);
+    aux_kernel<<<1, (L + 31) / 32 * 32, smem, s>>>(L, dt, state, state + L, state + 2 * L, state + 3 * L, state + 4 * L,
+                                                   state + 5 * L, coef, vals, nvals, s0, nsteps, Etab, Htab);
+    return 1;
+  }
+  if (nsteps <= 2) {
+    aux_long_kernel<<<1, 1024, 0, s>>>(L, dt, state, state + L, state + 2 * L, state + 3 * L, state + 4 * L, state + 5 * L,
+                                       coef, vals, nvals, s0, nsteps, Etab, Htab);
+    return 1;
+  }
+  const int n = 2 * ((nsteps + 2 * kAuxSteps - 1) / (2 * kAuxSteps));
+  double* const copy[2] = {state, state + 6 * static_cast<long long>(L)};
+  for (int q = 0; q < n; q++) {
+    const int at = static_cast<int>(static_cast<long long>(nsteps) * q / n);
+    const int T = static_cast<int>(static_cast<long long>(nsteps) * (q + 1) / n) - at;
+    launch_chained(aux_window_kernel, dim3(window_tiles(L, kAuxWin, kAuxWin - 2 * T)), dim3(32), 0, s, L, dt, copy[q & 1],
+                   copy[1 - (q & 1)], coef, vals, nvals, s0, T, at, Etab, Htab);
+  }
+  return n;
 }
 
 }  // namespace fdtdb

@@ -45,8 +45,7 @@ def test_groups_along_rows_match_the_flat_sweeps(fdtd, nx, ny, nz):
 
 @pytest.mark.parametrize("ncells", [950, 974, 975, 1500, 1998, 1999, 2300])
 def test_aux_grid_lengths_match_oracle(fdtd, oracle, ncells):
-    """Aux grids of ncells + 50 cells: one, two cells per thread, then the
-    state in memory; FP64, so the fields equal the oracle's within 1e-12."""
+    """Aux grids of ncells + 50 cells: a cell per thread up to 1024, then windows; FP64, so the fields equal the oracle's within 1e-12."""
     p = copy.deepcopy(scenarios.tm_tfsf_reference_polarisation())
     p.tfsf.aux_ncells = ncells
     # the incident wave starts at the aux grid's low end: bring the box there
@@ -55,6 +54,26 @@ def test_aux_grid_lengths_match_oracle(fdtd, oracle, ncells):
     g = fdtd.Grid.from_problem(p, "f64")
     g.step(p.steps // 2)
     g.step(p.steps - p.steps // 2)
+    E, H, _, _ = mode_fields(p.mode)
+    for n in E + H:
+        assert rel_l2(g.get(n), o.get(n)) <= 1e-12, n
+
+
+@pytest.mark.parametrize("ncells", [975, 976, 1037, 1038, 1039, 1198, 1200, 2030, 6000])
+@pytest.mark.parametrize("calls", [(64, 1, 2, 3), (5, 63, 2, 65)])
+def test_aux_windows_match_oracle(fdtd, oracle, ncells, calls):
+    """Rows of more than 1024 cells are stepped in windows of 128 cells: lengths
+    where the last window ends on the row's last cell and one to each side, calls
+    that split into one to 32 steps per launch, single steps between them; FP64,
+    so the fields equal the oracle's within 1e-12."""
+    p = copy.deepcopy(scenarios.tm_tfsf_reference_polarisation())
+    p.tfsf.aux_ncells = ncells
+    p.tfsf.origin = (p.tfsf.origin[0] + (ncells + 50) / 2 - 40.0, *p.tfsf.origin[1:]) if p.tfsf.k[0] else p.tfsf.origin
+    p.steps = sum(calls)
+    o = oracle.run_oracle(p)
+    g = fdtd.Grid.from_problem(p, "f64")
+    for n in calls:
+        g.step(n)
     E, H, _, _ = mode_fields(p.mode)
     for n in E + H:
         assert rel_l2(g.get(n), o.get(n)) <= 1e-12, n
