@@ -4,8 +4,10 @@
 // an even number of launches).
 //
 // What bounded a small FP64 grid was the chain of launches (256 x 256: 7 us per
-// step in four launches); what bounds a window is its FP64 arithmetic, the
-// reference's IEEE divisions among it. A thread holds two neighbouring columns
+// step in four launches); what bounds a window is the chain of a step through
+// shared memory and two barriers (a scheduler issues on 46% of cycles; waits on
+// shared memory 3.3, fixed latencies 2.5, barriers 2.0 cycles per issue) and its
+// instructions, the reference's IEEE divisions among them. A thread holds two neighbouring columns
 // of one row, so that the loop stays within the instruction cache (two rows per
 // thread, with every division in line, stalled 3.5 cycles per issue on it); 32
 // warps at 64 registers take one window per SM. The CPML integrators and the P and J of dispersive cells

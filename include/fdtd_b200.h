@@ -217,9 +217,9 @@ int fdtd_step(fdtd_grid* g, int nsteps, void* stream);
 /* 2D grids take calls of two steps or more in windows: several steps per
  * launch, from one copy of the state into another (the grid holds a second
  * copy of what a step changes, and per-cell material factors). FP32 grids do
- * without poles, mu_r != 1 and TFSF planes; FP64 grids with one mu_r, BD1, at
- * most one pole (TE) or two (TM) and 32 of sources, boxes and twice the TFSF
- * planes; both without boundary conditions and DFT of surface quantities.
+ * without mu_r != 1; FP64 grids with one mu_r, BD1, at most one pole (TE) or
+ * two (TM) and 32 of sources, boxes and twice the TFSF planes; both without
+ * boundary conditions and DFT of surface quantities.
  * Results are those of one launch per half step, which
  * fdtd_set_sweep_kernel(g, FDTD_SWEEP_REGS) brings back, and which a grid
  * keeps whose second copy finds no device memory. */
