@@ -3452,6 +3452,28 @@ static int adj_enqueue_segment(fdtd_adjoint* a, const FusedArgs& fa, const AdjAr
   return FDTD_OK;
 }
 
+// Why the adjoint does not take this grid (null: it does): its reversed steps
+// know no planes, poles, boundary images or mu_r.
+static const char* adj_grid_unsupported(const fdtd_grid* g) {
+  if (!g->planes.empty()) return "the adjoint takes grids without TFSF planes";
+  if (g->max_poles != 0) return "the adjoint takes non-dispersive materials";
+  if (g->bcs.n > 0) return "the adjoint takes grids without boundary conditions";
+  for (auto& m : g->mats)
+    if (m.mu_r != 1.0) return "the adjoint takes mu_r = 1";
+  return nullptr;
+}
+
+// The same for the box of the design cells (the CPML slabs laid out)
+static const char* adj_design_unsupported(const fdtd_grid* g, const int* lo, const int* hi) {
+  for (int d = 0; d < 2; d++)
+    for (int x = lo[d]; x <= hi[d]; x++)
+      if (slab_index(g->slab[d], x) >= 0) return "design box must lie outside the CPML";
+  for (const auto& sh : g->srcs)
+    if (sh.target == 1 && sh.i >= lo[0] && sh.i <= hi[0] && sh.j >= lo[1] && sh.j <= hi[1])
+      return "D-target sources inside the design box are not supported";
+  return nullptr;
+}
+
 extern "C" {
 
 int fdtd_adjoint_create(fdtd_grid* g, const int* probe_lo, const int* probe_hi, double freq, const int* design_lo,
@@ -3460,11 +3482,7 @@ int fdtd_adjoint_create(fdtd_grid* g, const int* probe_lo, const int* probe_hi, 
   if (!g->f32 || g->d.mode != FDTD_TM)
     return fail(FDTD_ERR_UNSUPPORTED, "the adjoint takes 2D TM grids of the FP32 fused method");
   if (g->t != 0) return fail(FDTD_ERR_INVALID, "the adjoint starts from a grid that has not been stepped");
-  if (!g->planes.empty()) return fail(FDTD_ERR_UNSUPPORTED, "the adjoint takes grids without TFSF planes");
-  if (g->max_poles != 0) return fail(FDTD_ERR_UNSUPPORTED, "the adjoint takes non-dispersive materials");
-  if (g->bcs.n > 0) return fail(FDTD_ERR_UNSUPPORTED, "the adjoint takes grids without boundary conditions");
-  for (auto& m : g->mats)
-    if (m.mu_r != 1.0) return fail(FDTD_ERR_UNSUPPORTED, "the adjoint takes mu_r = 1");
+  if (const char* why = adj_grid_unsupported(g)) return fail(FDTD_ERR_UNSUPPORTED, why);
   if (ckpt_every < 1 || ckpt_every > 4096) return fail(FDTD_ERR_INVALID, "ckpt_every must be 1..4096");
   {
     const int prc = ensure_pml(g);
@@ -3476,13 +3494,8 @@ int fdtd_adjoint_create(fdtd_grid* g, const int* probe_lo, const int* probe_hi, 
   for (int d = 0; d < 2; d++) {
     if (design_lo[d] > design_hi[d] || design_lo[d] < 1 || design_hi[d] > g->n[d] - 2)
       return fail(FDTD_ERR_INVALID, "design box must be a non-empty box of interior cells");
-    for (int x = design_lo[d]; x <= design_hi[d]; x++)
-      if (slab_index(g->slab[d], x) >= 0) return fail(FDTD_ERR_UNSUPPORTED, "design box must lie outside the CPML");
   }
-  for (const auto& sh : g->srcs)
-    if (sh.target == 1 && sh.i >= design_lo[0] && sh.i <= design_hi[0] && sh.j >= design_lo[1] &&
-        sh.j <= design_hi[1])
-      return fail(FDTD_ERR_UNSUPPORTED, "D-target sources inside the design box are not supported");
+  if (const char* why = adj_design_unsupported(g, design_lo, design_hi)) return fail(FDTD_ERR_UNSUPPORTED, why);
   CK(cudaSetDevice(g->d.device));
   const int lo3[3] = {probe_lo[0], probe_lo[1], 0}, hi3[3] = {probe_hi[0], probe_hi[1], 0};
   int handle = -1;
@@ -3522,7 +3535,17 @@ int fdtd_adjoint_forward(fdtd_adjoint* a, int nsteps, double* J) try {
   if (nsteps < 1) return fail(FDTD_ERR_INVALID, "nsteps < 1");
   fdtd_grid* g = a->g;
   if (g->t != 0) return fail(FDTD_ERR_INVALID, "the grid was stepped after the adjoint was created");
+  // t is still 0 after an E half step (step_impl refuses it; the stored path
+  // does not pass through there)
+  if (g->next_half != 0 || g->half_split) return fail(FDTD_ERR_INVALID, "an E half step was taken without its H half");
+  // the grid may have changed since it was created
+  if (const char* why = adj_grid_unsupported(g)) return fail(FDTD_ERR_UNSUPPORTED, why);
   CK(cudaSetDevice(g->d.device));
+  {
+    const int prc = ensure_pml(g);
+    if (prc) return prc;
+  }
+  if (const char* why = adj_design_unsupported(g, a->dlo, a->dhi)) return fail(FDTD_ERR_UNSUPPORTED, why);
   if (g->dirty_dft) {
     int rc = rebuild_dft(g);
     if (rc) return rc;

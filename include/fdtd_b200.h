@@ -411,7 +411,8 @@ int fdtd_batch_error_flags(fdtd_batch* b, int* flags);
  * |X|^2, X the running DFT of Ez at `freq` (cycles per step, samples as
  * fdtd_add_dft). The grid must be unstepped, without TFSF planes or
  * dispersive materials; the design box must lie outside the CPML and hold no
- * D-target source. create adds the probe DFT region to the grid. forward
+ * D-target source; create and forward both check it. A pending E half step
+ * is FDTD_ERR_INVALID. create adds the probe DFT region to the grid. forward
  * steps the grid nsteps times and returns J, keeping one FP32 value per
  * design cell and step where these take at most a sixteenth of the device's
  * memory (and the grid takes its steps in windows, see fdtd_step), else
