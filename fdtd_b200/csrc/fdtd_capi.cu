@@ -3339,11 +3339,34 @@ static int adjoint_capture_step(fdtd_adjoint* a, long long t, cudaStream_t s) {
   return launch_adjoint_capture(aa, fa.H[0], fa.H[1], a->d_dt + t * aa.ndesign, s);
 }
 
+// elements of the adjoint state of the windows: aez, ahx, ahy, the integrators
+static void adj_win_elems(const fdtd_grid* g, size_t (&elems)[7]) {
+  const size_t fe = static_cast<size_t>(field_elems(g));
+  const size_t sx = static_cast<size_t>(g->n[1]) * g->slab[0].W4, sy = static_cast<size_t>(g->slab[1].W) * rowlen(g);
+  const size_t e[7] = {fe, fe, fe, sy, sx, sx, sy};
+  std::copy(e, e + 7, elems);
+}
+
+// gives back every buffer of the handle
+static void adj_release(fdtd_adjoint* a) {
+  for (void* p : a->buf.allocs) cudaFree(p);
+  a->buf.allocs.clear();
+  a->d_dt = a->d_force = a->d_ie = nullptr;
+  a->d_X = a->d_grad = nullptr;
+  for (auto& c : a->win)
+    for (auto& p : c) p = nullptr;
+}
+
 // The forward of a grid that takes its steps in windows, keeping d_t of every
 // design cell: the backward then needs neither the forward's states nor its
 // steps again. *done says whether it ran: not for a grid that keeps the
-// launches per half step, nor where the terms would take more than a
-// sixteenth of the device's memory (checkpoints and recomputation then).
+// launches per half step, nor where the terms (or the probes' values) would
+// take more than a sixteenth of the device's memory, or the whole of it more
+// than 8 times what the checkpoints every ckpt_every steps take (so that the
+// caller's choice of ckpt_every still bounds the memory; 512 x 512 cells with a
+// 128 x 128 design box, 4000 steps, every 64: 269 MB against 232), nor where
+// it does not fit. All that the backward needs is laid out here, so that it
+// cannot run out of memory where the checkpoints would have fit.
 static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
   fdtd_grid* g = a->g;
   *done = false;
@@ -3352,14 +3375,26 @@ static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
   if (rc || !g->win_ok) return rc;
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b));
-  const size_t bytes = static_cast<size_t>(nsteps) * adj_design(a) * sizeof(float);
+  const size_t nd = static_cast<size_t>(adj_design(a)), fe = static_cast<size_t>(field_elems(g));
+  const size_t bytes = static_cast<size_t>(nsteps) * nd * sizeof(float);
   const size_t np = static_cast<size_t>(a->phi[0] - a->plo[0] + 1) * (a->phi[1] - a->plo[1] + 1);
   const size_t fbytes = static_cast<size_t>(nsteps) * np * sizeof(float);
-  if (bytes > total_b / 16 || fbytes > total_b / 16) return FDTD_OK;
+  size_t elems[7], state = 0, checkpoint = 0;
+  adj_win_elems(g, elems);
+  for (size_t e : elems) state += 2 * e * sizeof(float);
+  for (const auto& st : grid_state(g)) checkpoint += st.second;
+  const size_t nckpt = (static_cast<size_t>(nsteps) + a->ckpt_every - 1) / a->ckpt_every;
+  const size_t checkpoints = checkpoint * (nckpt + 1) + (static_cast<size_t>(a->ckpt_every) * nd + 7 * fe) * sizeof(float);
+  if (bytes > total_b / 16 || fbytes > total_b / 16 || bytes + fbytes + state > 8 * checkpoints) return FDTD_OK;
   rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_dt), bytes);
   if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_force), fbytes);
+  if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_X), np * 2 * sizeof(double));
+  if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_ie), fe * sizeof(float));
+  if (!rc) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_grad), nd * sizeof(double));
+  for (auto& c : a->win)
+    for (int q = 0; q < 7 && !rc; q++) rc = adj_alloc(a, reinterpret_cast<void**>(&c[q]), elems[q] * sizeof(float));
   if (rc) {
-    a->d_dt = nullptr;
+    adj_release(a);
     return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
   }
   if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
@@ -3374,18 +3409,11 @@ static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
 static int adj_backward_stored(fdtd_adjoint* a, const FusedArgs& fa) {
   fdtd_grid* g = a->g;
   cudaStream_t s = g->stream;
-  const size_t fe = static_cast<size_t>(field_elems(g));
-  const size_t sx = static_cast<size_t>(g->n[1]) * g->slab[0].W4, sy = static_cast<size_t>(g->slab[1].W) * rowlen(g);
-  const size_t elems[7] = {fe, fe, fe, sy, sx, sx, sy};
+  size_t elems[7];
+  adj_win_elems(g, elems);
   const int np = (a->phi[0] - a->plo[0] + 1) * (a->phi[1] - a->plo[1] + 1);
-  for (int c = 0; c < 2; c++)
-    for (int q = 0; q < 7; q++) {
-      if (!a->win[c][q]) {
-        const int rc = adj_alloc(a, reinterpret_cast<void**>(&a->win[c][q]), elems[q] * sizeof(float));
-        if (rc) return rc;
-      }
-      CK(cudaMemsetAsync(a->win[c][q], 0, std::max<size_t>(elems[q], 4) * sizeof(float), s));
-    }
+  for (auto& c : a->win)
+    for (int q = 0; q < 7; q++) CK(cudaMemsetAsync(c[q], 0, std::max<size_t>(elems[q], 4) * sizeof(float), s));
   AdjWinArgs w;
   memset(&w, 0, sizeof(w));
   const WinArgs& f = g->win;
@@ -3571,7 +3599,7 @@ int fdtd_adjoint_forward(fdtd_adjoint* a, int nsteps, double* J) try {
     if (rc) return rc;
   }
   const DftH& r = g->dfts[a->dft];
-  rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_X), static_cast<size_t>(r.npts) * 2 * sizeof(double));
+  if (!a->d_X) rc = adj_alloc(a, reinterpret_cast<void**>(&a->d_X), static_cast<size_t>(r.npts) * 2 * sizeof(double));
   if (rc) return rc;
   CK(cudaMemcpyAsync(a->d_X, r.d_acc, r.npts * 2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
   std::vector<double> X(static_cast<size_t>(r.npts) * 2);

@@ -415,8 +415,10 @@ int fdtd_batch_error_flags(fdtd_batch* b, int* flags);
  * is FDTD_ERR_INVALID. create adds the probe DFT region to the grid. forward
  * steps the grid nsteps times and returns J, keeping one FP32 value per
  * design cell and step where these take at most a sixteenth of the device's
- * memory (and the grid takes its steps in windows, see fdtd_step), else
- * checkpointing the state every ckpt_every steps; backward reverses the steps
+ * memory and, with the rest of what backward needs, at most 8 times what the
+ * checkpoints take, and fit (and the grid takes its steps in windows, see
+ * fdtd_step), else checkpointing the state every ckpt_every steps (always with
+ * FDTD_SWEEP_REGS); backward reverses the steps
  * from the kept values, or recomputes each segment from its checkpoint and
  * reverses it, leaves the grid in its post-forward state and writes
  * dJ/deps_r of every design cell (x fastest) to the host array grad. One
