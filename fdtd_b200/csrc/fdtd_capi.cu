@@ -230,6 +230,7 @@ struct fdtd_grid {
   unsigned* d_eh = nullptr;  // one-launch step: [0] epoch, then the E tile flags
   long long eh_words = 0;
   long long version = 0;        // bumped by every change a captured graph would bake in
+  long long psi_layouts = 0;    // times the CPML integrators were laid out
   long long graph_version = -1;
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0;
@@ -400,6 +401,7 @@ int alloc_psi(fdtd_grid* g) {
         }
       }
   for (int a = 0; a < 3; a++) g->slab[a] = make_slab(g->n[a], g->pml[a][0], g->pml[a][1]);
+  g->psi_layouts++;
   for (int ft = 0; ft < 2; ft++)
     for (int I = 0; I < 3; I++) {
       const bool has = ft == 0 ? hasE(g->d.mode, I) : hasH(g->d.mode, I);
@@ -3265,6 +3267,7 @@ struct fdtd_adjoint {
   int dft = -1;
   long long nsteps = 0;
   bool forwarded = false;
+  long long psi_layouts = 0;  // the grid's at the forward
   std::vector<std::pair<void*, size_t>> state;
   size_t state_bytes = 0;
   int nckpt = 0;
@@ -3416,7 +3419,7 @@ static int adj_backward_stored(fdtd_adjoint* a, const FusedArgs& fa) {
     for (int q = 0; q < 7; q++) CK(cudaMemsetAsync(c[q], 0, std::max<size_t>(elems[q], 4) * sizeof(float), s));
   AdjWinArgs w;
   memset(&w, 0, sizeof(w));
-  const WinArgs& f = g->win;
+  const WinArgs f = window_args(g);
   w.nx = f.nx;
   w.ny = f.ny;
   w.pitch = f.pitch;
@@ -3610,6 +3613,7 @@ int fdtd_adjoint_forward(fdtd_adjoint* a, int nsteps, double* J) try {
   a->J = sum;
   a->nsteps = nsteps;
   a->forwarded = true;
+  a->psi_layouts = g->psi_layouts;
   *J = sum;
   return FDTD_OK;
 } catch (...) {
@@ -3621,6 +3625,8 @@ int fdtd_adjoint_backward(fdtd_adjoint* a, double* grad) try {
   if (!a->forwarded) return fail(FDTD_ERR_INVALID, "run fdtd_adjoint_forward first");
   fdtd_grid* g = a->g;
   if (g->t != a->nsteps) return fail(FDTD_ERR_INVALID, "the grid was stepped after the adjoint forward");
+  // the checkpoints hold the old integrators' addresses, the kept terms' sizes theirs
+  if (g->psi_layouts != a->psi_layouts) return fail(FDTD_ERR_INVALID, "the CPML was laid out anew after the adjoint forward");
   CK(cudaSetDevice(g->d.device));
   cudaStream_t s = g->stream;
   const size_t fe = static_cast<size_t>(field_elems(g));

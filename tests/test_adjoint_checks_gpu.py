@@ -69,3 +69,16 @@ def test_forward_refuses_what_create_refuses(fdtd, kind, change):
     with pytest.raises(fdtd.FdtdError) as e:
         adj.forward(70)
     assert e.value.code == UNSUPPORTED and g.step_count == 0
+
+
+@pytest.mark.parametrize("kind", ["auto", "regs"])
+def test_backward_refuses_a_cpml_laid_out_anew(fdtd, kind):
+    """A CPML set after the forward, and its integrators laid out (reading one
+    does): the checkpoints and the adjoint state belong to the old ones."""
+    _, g, adj = _created(fdtd, kind)
+    adj.forward(70)
+    g.set_pml(0, 0, 3)
+    g.get(fdtd.PSI_NAMES[2 * 3 + 0])
+    with pytest.raises(fdtd.FdtdError) as e:
+        adj.backward()
+    assert e.value.code == INVALID
