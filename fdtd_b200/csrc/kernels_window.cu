@@ -193,6 +193,28 @@ __device__ __forceinline__ void sample_regions(const Region* reg, unsigned set, 
   }
 }
 
+// Writes the launch's T samples of the thread's cells on the outer ring again,
+// from the ring's values in memory, which it keeps: their registers became NaN
+// next to a cell that is not finite. Out of line and at the kernel's end, where
+// nothing else is live: next to no thread comes here.
+template <bool TE, int R, class Sh>
+__device__ __noinline__ void sample_ring(const WinArgs& a, const Sh& sh, int x0, int y0, int T, int from, int slot) {
+  const int lane = threadIdx.x & 31, row0 = (threadIdx.x >> 5) * R;
+  for (int h = 0; h < 2; h++)
+    for (int k = 0; k < sh.nreg[h]; k++) {
+      const Region& g = sh.reg[h][k];
+      // the components' places in a.f: TE Ex, Ey, Hz, TM Ez, Hx, Hy
+      const float* f = a.f[from][h == 0 ? (TE ? g.comp : 0) : (TE ? 2 : 1 + g.comp)];
+      for (int w = max(g.lo[1], row0); w <= min(g.hi[1], row0 + R - 1); w++)
+        for (int l = max(g.lo[0], 2 * lane); l <= min(g.hi[0], 2 * lane + 1); l++) {
+          const int i = x0 + l, j = y0 + w;
+          if (i > 0 && i < a.nx - 1 && j > 0 && j < a.ny - 1) continue;
+          const float v = __ldcg(f + j * static_cast<long long>(a.pitch) + i);
+          for (int st = 0; st < T; st++) g.out[(slot + st) * a.dft_pts[h] + static_cast<long long>(w) * g.ex + l] = v;
+        }
+    }
+}
+
 // Grids with poles or TFSF planes (EXT, kernels of their own, so that the others
 // keep their registers). What bounded them was, as for the rest, the chain of
 // launches: 9.9 us a step at 160 x 96 TE with Drude cells, 18.3 with TFSF planes
@@ -274,9 +296,10 @@ struct WinSpan {
 
 // One window, T steps. GEN: the window touches the outer ring, the CPML, a
 // source or a DFT region; otherwise every cell is interior with the plain
-// coefficients and nothing else acts on it.
+// coefficients and nothing else acts on it. True where a thread's samples of the
+// outer ring are lost (sample_ring).
 template <int MODE, bool XFIRST, bool GEN, bool CAP, int NW, int R, class Ext>
-__device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] const Ext& x, [[maybe_unused]] const ExtShared* es,
+__device__ __forceinline__ bool window_run(const WinArgs& a, [[maybe_unused]] const Ext& x, [[maybe_unused]] const ExtShared* es,
                                            Shared<NW, R>& sh, float* psi, const WinSpan& sp, int T,
                                            int from, int slot, long long t0, pair_t (&f0)[R], pair_t (&f1)[R], pair_t (&f2)[R],
                                            pair_t (&ie)[R]) {
@@ -299,7 +322,8 @@ __device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] co
   // GEN. A cell of the outer ring (or beyond the grid) keeps its value: its
   // 1/eps is zero in the E half and its factor of the H half too; rows
   // outside the interior skip the H half. (A ring cell next to a non-finite
-  // one would become NaN here; its own value is restored at the end.)
+  // one becomes NaN here; it is sampled and written back as it was, and the
+  // interior cells that see it are non-finite already.)
   const bool ok0 = !GEN || (c0 >= 1 && c0 <= a.nx - 2), ok1 = !GEN || c0 + 1 <= a.nx - 2;
   const pair_t minus = GEN ? pack(ok0 ? -1.f : 0.f, ok1 ? -1.f : 0.f) : both(-1.f);
   int xs = -1;  // the columns' place in the aligned x slab rows, or -1
@@ -672,8 +696,20 @@ __device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] co
     __syncthreads();
   }
 
+  // a sampled cell of the ring once NaN stays so for the launch (a batch samples nothing)
+  bool lost = false;
+  if (GEN && XFIRST && __builtin_expect((reg_e | reg_h) != 0, 0)) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const float2 u[3] = {unpack(f0[r]), unpack(f1[r]), unpack(f2[r])};
+      const bool row = rows_in >> r & 1;
+#pragma unroll
+      for (int q = 0; q < 3; q++) lost = lost || (!(row && ok0) && isnan(u[q].x)) || (!(row && ok1) && isnan(u[q].y));
+    }
+  }
+
   // the exact cells, into the other copy of the state
-  if (c0 < sp.ox0 || c0 >= sp.ox1) return;
+  if (c0 < sp.ox0 || c0 >= sp.ox1) return lost;
   const int to = 1 - from;
   // a pair with the halves that hold no interior cell as they were
   auto put = [&](const float* was, float* now, long long at, pair_t v, bool row_ok) {
@@ -693,7 +729,7 @@ __device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] co
     put(a.f[from][1], a.f[to][1], c, f1[r], in);
     put(a.f[from][2], a.f[to][2], c, f2[r], in);
   }
-  if (!GEN) return;
+  if (!GEN) return lost;
 #pragma unroll 1
   for (int r = 0; r < R; r++) {
     const int j = j0 + r;
@@ -724,6 +760,7 @@ __device__ __forceinline__ void window_run(const WinArgs& a, [[maybe_unused]] co
       }
     }
   }
+  return lost;
 }
 
 // The window of tile `tile` of a grid: first cell, owned cells, what acts in
@@ -836,14 +873,16 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, const Ext& x, ExtS
   bool plain = sp.x0 >= a.plain[0][0] && sp.x0 + kWinCols - 1 <= a.plain[0][1] && sp.y0 >= a.plain[1][0] &&
                      sp.y0 + rows - 1 <= a.plain[1][1] && sh.nentry + sh.nreg[0] + sh.nreg[1] == 0;
   if constexpr (EXT) plain = plain && !poles && es->nplane[0] + es->nplane[1] == 0;
+  bool lost = false;
   if (plain) window_run<MODE, XFIRST, false, CAP, NW, R>(a, x, es, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
-  else window_run<MODE, XFIRST, true, CAP, NW, R>(a, x, es, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
+  else lost = window_run<MODE, XFIRST, true, CAP, NW, R>(a, x, es, sh, psi, sp, T, from, slot, t0, f0, f1, f2, ie);
   // the soft sources' last values, by the window that owns the source cell
   if (tid < a.nsrc) {
     const SourceDev& q = a.src[tid];
     if ((q.target == 0 || q.target == 2) && q.i >= sp.ox0 && q.i < sp.ox1 && q.j >= sp.oy0 && q.j < sp.oy1)
       a.src_last[1 - from][tid] = table_value(q.vals, q.nvals, t0 + T - 1);
   }
+  if (XFIRST && __builtin_expect(lost, 0)) sample_ring<MODE == kTE, R>(a, sh, sp.x0, sp.y0, T, from, slot);
 }
 
 template <int MODE, bool CAP, int NW, int R>
