@@ -1924,6 +1924,9 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
   WinArgs wa = g->win;
   if (adj) adjoint_capture_args(adj, wa);
   const bool dft = !g->dfts.empty();
+  bool ring = false;  // a region holds cells of the outer ring
+  for (const auto& r : g->dfts)
+    for (int d = 0; d < 2; d++) ring = ring || r.lo[d] == 0 || r.hi[d] == g->n[d] - 1;
   int rows = kWinRows;
   // with Lorentz poles a window of 64 rows is more than an SM's shared memory;
   // with Drude poles one fits instead of two and is still the faster (3000 x
@@ -1954,6 +1957,7 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
       g->launches += g->f32 ? launch_window(g->d.mode, wa, ext, rows, t, at, q & 1, g->dft_pending + at, s)
                             : launch_window64(g->d.mode, g->win64, t, at, q & 1, g->dft_pending + at, s);
     }
+    if (adj && ring) g->launches += launch_window_ring(g->d.mode, wa, g->dft_maxpts, g->dft_pending, n, s);
     g->launches += launch_steps_advance(g->ctrl, n, s);
     if (dft) {
       g->dft_pending += n;

@@ -696,9 +696,11 @@ __device__ __forceinline__ bool window_run(const WinArgs& a, [[maybe_unused]] co
     __syncthreads();
   }
 
-  // a sampled cell of the ring once NaN stays so for the launch (a batch samples nothing)
+  // a sampled cell of the ring once NaN stays so for the launch (a batch samples
+  // nothing; the adjoint's forward has launch_window_ring: the check cost its
+  // kernel 4%)
   bool lost = false;
-  if (GEN && XFIRST && __builtin_expect((reg_e | reg_h) != 0, 0)) {
+  if (GEN && XFIRST && !CAP && __builtin_expect((reg_e | reg_h) != 0, 0)) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const float2 u[3] = {unpack(f0[r]), unpack(f1[r]), unpack(f2[r])};
@@ -882,7 +884,7 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, const Ext& x, ExtS
     if ((q.target == 0 || q.target == 2) && q.i >= sp.ox0 && q.i < sp.ox1 && q.j >= sp.oy0 && q.j < sp.oy1)
       a.src_last[1 - from][tid] = table_value(q.vals, q.nvals, t0 + T - 1);
   }
-  if (XFIRST && __builtin_expect(lost, 0)) sample_ring<MODE == kTE, R>(a, sh, sp.x0, sp.y0, T, from, slot);
+  if (XFIRST && !CAP && __builtin_expect(lost, 0)) sample_ring<MODE == kTE, R>(a, sh, sp.x0, sp.y0, T, from, slot);
 }
 
 template <int MODE, bool CAP, int NW, int R>
@@ -949,6 +951,20 @@ __global__ void window_cells_kernel(const __grid_constant__ FusedArgs a, unsigne
   disp[c] = static_cast<unsigned short>(n == 0 ? 0 : (n < 0 ? 1 : n) << 14 | mid);
 }
 
+// the samples of the outer ring's cells in slots slot .. slot + n - 1, one region
+// per blockIdx.y, a thread per point
+__global__ void __launch_bounds__(256) window_ring_kernel(const __grid_constant__ WinArgs a, int mode, int h, int slot, int n) {
+  const DftRegionDev& g = a.reg[h][blockIdx.y];
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q >= g.npts) return;
+  const int i = g.lo[0] + q % g.ext[0], j = g.lo[1] + q / g.ext[0];
+  if (i > 0 && i < a.nx - 1 && j > 0 && j < a.ny - 1) return;
+  const bool te = mode == kTE;
+  const float* f = a.f[0][h == 0 ? (te ? g.comp : 0) : (te ? 2 : 1 + g.comp)];
+  const float v = f[j * static_cast<long long>(a.pitch) + i];
+  for (int s = slot; s < slot + n; s++) a.dft_buf[h][s * a.dft_pts[h] + g.pt_off + q] = v;
+}
+
 size_t ext_bytes(int mode, const WinExt& x, int rows) {
   const size_t cells = static_cast<size_t>(kWinCols) * rows;
   return ext_arrays(mode, x) * cells * sizeof(float) + (x.np > 0 ? cells * sizeof(unsigned short) : 0);
@@ -970,6 +986,16 @@ void window_ext_go(F fn, int mode, int n, cudaStream_t st, const WinArgs& a, con
 int launch_window_cells(const FusedArgs& a, unsigned short* disp, cudaStream_t s) {
   window_cells_kernel<<<dim3((a.pitch + 31) / 32, (a.ny + 7) / 8), dim3(32, 8), 0, s>>>(a, disp);
   return 1;
+}
+
+int launch_window_ring(int mode, const WinArgs& a, const long long (&max_pts)[2], int slot, int n, cudaStream_t s) {
+  int launches = 0;
+  for (int h = 0; h < 2; h++) {
+    if (a.nreg[h] == 0) continue;
+    window_ring_kernel<<<dim3(static_cast<unsigned>((max_pts[h] + 255) / 256), a.nreg[h]), 256, 0, s>>>(a, mode, h, slot, n);
+    launches++;
+  }
+  return launches;
 }
 
 int launch_window(int mode, const WinArgs& a, const WinExt* x, int rows, int T, int s, int from, int slot, cudaStream_t st) {

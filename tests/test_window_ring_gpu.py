@@ -42,3 +42,28 @@ def test_non_finite_cells(fdtd, prec, mode, npml, value, cell):
         assert np.array_equal(np.isfinite(a), np.isfinite(b)), q
         ok = np.isfinite(a)
         assert np.array_equal(a[ok], b[ok]) and np.any(a[ok]), q
+
+
+def test_adjoint_forward_of_a_non_finite_grid(fdtd):
+    """The same for the forward of the stored adjoint, a spectrum over the whole
+    grid beside the probe's."""
+    nx, ny = 90, 70
+    out = []
+    for kind in ("auto", "regs"):
+        p = P.Problem(P.TM, (nx, ny, 1), 1e-6, P.courant_dt(1e-6, 0.98 / np.sqrt(2.0)))
+        p.dfts.append(P.DFTRegion(2, (0, 0, 0), (nx - 1, ny - 1, 0), [0.02]))
+        p.dfts.append(P.DFTRegion(4, (0, 5, 0), (nx - 1, 5, 0), [0.02]))
+        g = fdtd.Grid.from_problem(p, "f32")
+        g.set_sweep_kernel(kind)
+        v = np.random.default_rng(0).normal(size=(1, ny, nx))
+        v[0, 3, 2] = np.inf
+        v[0, 0, :] = v[0, -1, :] = v[0, :, 0] = 0.25
+        g.set("Ez", v)
+        adj = fdtd.Adjoint(g, (70, 30), (70, 33), 0.05, (40, 30), (50, 40), 64)
+        J = adj.forward(12)
+        out.append([np.array(J), g.get("Ez"), g.get("Hy"), g.dft(0), g.dft(1)])
+        adj.close()
+    for q, (a, b) in enumerate(zip(*out)):
+        ok = np.isfinite(a)
+        assert np.array_equal(ok, np.isfinite(b)), q
+        assert np.array_equal(a[ok], b[ok]) and np.any(a[ok]), q
