@@ -1957,7 +1957,7 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
       g->launches += g->f32 ? launch_window(g->d.mode, wa, ext, rows, t, at, q & 1, g->dft_pending + at, s)
                             : launch_window64(g->d.mode, g->win64, t, at, q & 1, g->dft_pending + at, s);
     }
-    if (adj && ring) g->launches += launch_window_ring(g->d.mode, wa, g->dft_maxpts, g->dft_pending, n, s);
+    if ((adj || ext) && ring) g->launches += launch_window_ring(g->d.mode, wa, g->dft_maxpts, g->dft_pending, n, s);
     g->launches += launch_steps_advance(g->ctrl, n, s);
     if (dft) {
       g->dft_pending += n;

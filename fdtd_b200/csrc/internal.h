@@ -353,7 +353,7 @@ inline int window_count(int nx, int ny, int rows, int T) {
 // (x: null, or what the grid's poles and TFSF planes need)
 int launch_window(int mode, const WinArgs& a, const WinExt* x, int rows, int T, int s, int from, int slot, cudaStream_t st);
 // the ring's samples of n steps in slots slot .. slot + n - 1, from the ring's
-// values (which it keeps), for windows that do not see to them themselves (a.cap)
+// values (which it keeps), for windows that do not see to them themselves (a.cap, poles, planes)
 int launch_window_ring(int mode, const WinArgs& a, const long long (&max_pts)[2], int slot, int n, cudaStream_t s);
 // the materials with poles of every cell
 int launch_window_cells(const FusedArgs& a, unsigned short* disp, cudaStream_t s);

@@ -697,10 +697,10 @@ __device__ __forceinline__ bool window_run(const WinArgs& a, [[maybe_unused]] co
   }
 
   // a sampled cell of the ring once NaN stays so for the launch (a batch samples
-  // nothing; the adjoint's forward has launch_window_ring: the check cost its
-  // kernel 4%)
+  // nothing; the adjoint's forward and EXT have launch_window_ring: the check cost
+  // their kernels 4%)
   bool lost = false;
-  if (GEN && XFIRST && !CAP && __builtin_expect((reg_e | reg_h) != 0, 0)) {
+  if (GEN && XFIRST && !CAP && !EXT && __builtin_expect((reg_e | reg_h) != 0, 0)) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const float2 u[3] = {unpack(f0[r]), unpack(f1[r]), unpack(f2[r])};
@@ -884,7 +884,7 @@ __device__ __forceinline__ void window_tile(const WinArgs& a, const Ext& x, ExtS
     if ((q.target == 0 || q.target == 2) && q.i >= sp.ox0 && q.i < sp.ox1 && q.j >= sp.oy0 && q.j < sp.oy1)
       a.src_last[1 - from][tid] = table_value(q.vals, q.nvals, t0 + T - 1);
   }
-  if (XFIRST && !CAP && __builtin_expect(lost, 0)) sample_ring<MODE == kTE, R>(a, sh, sp.x0, sp.y0, T, from, slot);
+  if (XFIRST && !CAP && !EXT && __builtin_expect(lost, 0)) sample_ring<MODE == kTE, R>(a, sh, sp.x0, sp.y0, T, from, slot);
 }
 
 template <int MODE, bool CAP, int NW, int R>

@@ -67,3 +67,30 @@ def test_adjoint_forward_of_a_non_finite_grid(fdtd):
         ok = np.isfinite(a)
         assert np.array_equal(ok, np.isfinite(b)), q
         assert np.array_equal(a[ok], b[ok]) and np.any(a[ok]), q
+
+
+@pytest.mark.parametrize("mode", [P.TE, P.TM], ids=["te", "tm"])
+def test_non_finite_cells_beside_poles(fdtd, mode):
+    """FP32 windows of a grid with Drude cells in its corner, where the value is."""
+    nx, ny = 90, 70
+    p = P.Problem(mode, (nx, ny, 1), 1e-6, P.courant_dt(1e-6, 0.98 / np.sqrt(2.0)))
+    p.materials.append(P.Material.drude(1.0, 0.25 / p.dt, 0.02 / p.dt))
+    p.ids = np.zeros((1, ny, nx), np.uint8)
+    p.ids[0, :12, :15] = 1
+    E, H, _, _ = mode_fields(mode)
+    for c in ([0, 1, 5] if mode == P.TE else [2, 3, 4]):
+        p.dfts.append(P.DFTRegion(c, (0, 0, 0), (nx - 1, ny - 1, 0), [0.02]))
+    v = np.random.default_rng(0).normal(size=(1, ny, nx))
+    v[0, 3, 2] = np.inf
+    v[0, 0, :] = v[0, -1, :] = v[0, :, 0] = 0.25
+    out = []
+    for kind in ("auto", "regs"):
+        g = fdtd.Grid.from_problem(p, "f32")
+        g.set_sweep_kernel(kind)
+        g.set(E[-1], v)
+        g.step(8)
+        out.append([g.get(n) for n in E + H] + [g.dft(h) for h in g.dft_handles])
+    for q, (a, b) in enumerate(zip(*out)):
+        ok = np.isfinite(a)
+        assert np.array_equal(ok, np.isfinite(b)), q
+        assert np.array_equal(a[ok], b[ok]) and np.any(a[ok]), q
