@@ -38,7 +38,7 @@ SOURCES = {
     "kernels_adjoint.cu": [],
     "fdtd_capi.cu": [],
 }
-HEADERS = ["internal.h", "fused3d_common.cuh", "pairs.cuh", "plain_tfsf.cuh", "quotient.cuh", os.path.join("..", "..", "include", "fdtd_b200.h")]
+HEADERS = ["internal.h", "fused3d_common.cuh", "pairs.cuh", "plain_tfsf.cuh", "quotient.cuh", "window_plan.h", os.path.join("..", "..", "include", "fdtd_b200.h")]
 
 
 def _newer(target: str, deps) -> bool:

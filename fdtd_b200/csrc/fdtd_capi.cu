@@ -21,6 +21,7 @@
 #include "../../include/fdtd_b200.h"
 #include "internal.h"
 #include "quotient.cuh"
+#include "window_plan.h"
 
 using namespace fdtdb;
 
@@ -205,7 +206,7 @@ struct fdtd_grid {
   int dft_pending = 0;    // samples in the buffers: the slot of the next one
   void** d_fieldptrs = nullptr;  // [E0,E1,E2,H0,H1,H2]
   Control* ctrl = nullptr;
-  int* d_flag = nullptr;
+  int* d_flag = nullptr;  // [0] a non-finite value, [2] and [3] blocks with poles
   char* h_stage = nullptr;  // two pinned chunks of kStageChunk bytes for large reads
   cudaEvent_t stage_ev[2]{};
   bool dirty_dft = true;
@@ -226,6 +227,17 @@ struct fdtd_grid {
   WinExt win_ext;            // FP32: what poles and TFSF planes need
   long long win_version = -1;
   bool win_ok = false;
+  // which stretches of steps go out in windows (window_plan), by their steps and
+  // whether a graph replays them, for the version they were planned for
+  long long plan_version = -1;
+  bool win_wanted = false;
+  bool win_always = false;  // fdtd_always_window
+  WindowCase win_case;
+  std::vector<WindowPlan> plans;
+  long long material_version = 0;  // bumped by every change of materials, ids or permittivities
+  long long share_version = -1;
+  double pole_share[2]{};
+  int sms = 148;
   TmaState* tma = nullptr;
   unsigned* d_eh = nullptr;  // one-launch step: [0] epoch, then the E tile flags
   long long eh_words = 0;
@@ -900,15 +912,80 @@ bool window_uniform(const fdtd_grid* g) {
   return !g->d_eps_map && ((!g->d_ids && !g->d_bids) || g->mats.size() == 1);
 }
 
+int ensure_window64(fdtd_grid* g);
+
+// The shares of the grid's cell blocks that hold poles (WindowCase::pole_share),
+// counted on the device once per change of the materials
+int ensure_pole_share(fdtd_grid* g) {
+  if (g->share_version == g->material_version) return FDTD_OK;
+  const bool all = g->max_poles != 0;
+  g->pole_share[0] = g->pole_share[1] = all ? 1.0 : 0.0;
+  if (all && (g->d_ids || g->d_bids)) {
+    unsigned* const counts = reinterpret_cast<unsigned*>(g->d_flag + 2);
+    unsigned n[2] = {0, 0};
+    CK(cudaMemsetAsync(counts, 0, sizeof(n), g->stream));
+    g->launches += g->f32 ? launch_pole_blocks(fused_args(g), counts, g->stream) : launch_pole_blocks(plain_args(g), counts, g->stream);
+    CK(cudaMemcpyAsync(n, counts, sizeof(n), cudaMemcpyDeviceToHost, g->stream));
+    CK(cudaStreamSynchronize(g->stream));
+    const double columns = (g->n[0] + 63) / 64;
+    g->pole_share[0] = n[0] / (columns * ((g->n[1] + 31) / 32));
+    g->pole_share[1] = n[1] / (columns * ((g->n[1] + 63) / 64));
+  }
+  g->share_version = g->material_version;
+  return FDTD_OK;
+}
+
+// What the plans of the grid's stretches depend on
+int ensure_plans(fdtd_grid* g) {
+  if (g->plan_version == g->version) return FDTD_OK;
+  g->win_wanted = window_wanted(g);
+  g->plans.clear();
+  if (g->win_wanted) {
+    const int rc = ensure_pole_share(g);
+    if (rc) return rc;
+    WindowCase& c = g->win_case;
+    c.f32 = g->f32;
+    c.te = g->d.mode == kTE;
+    c.nx = g->n[0];
+    c.ny = g->n[1];
+    const bool lorentz = std::any_of(g->mats.begin(), g->mats.end(), [](const fdtd_material& m) { return m.kind == FDTD_LORENTZ; });
+    c.poles = g->max_poles == 0 ? 0 : !lorentz ? 1 : 1 + std::abs(g->max_poles);
+    for (int q = 0; q < 2; q++) c.pole_share[q] = g->pole_share[q];
+    c.planes = static_cast<int>(g->planes.size());
+    c.gathers = (g->ndft[0] > 0) + (g->ndft[1] > 0);
+    c.boxes = static_cast<int>(g->boxes.size());
+    c.sms = g->sms;
+    g->plans.assign(2 * (kDftChunk + 1), WindowPlan{});
+  }
+  g->plan_version = g->version;
+  return FDTD_OK;
+}
+
+// The plan of a stretch of n <= kDftChunk steps (after ensure_plans)
+const WindowPlan& plan_of(fdtd_grid* g, int n, bool graph) {
+  WindowPlan& p = g->plans[n + (graph ? kDftChunk + 1 : 0)];
+  if (p.us == 0.0) {
+    g->win_case.graph = graph;
+    p = window_plan(g->win_case, n);
+    if (g->win_always) p.windows = p.launches > 0;
+  }
+  return p;
+}
+
+// Whether any stretch of a call of nsteps steps goes out in windows
+bool takes_windows(fdtd_grid* g, int nsteps) {
+  if (!g->win_wanted) return false;
+  const int rest = nsteps % kDftChunk;
+  return (nsteps >= kDftChunk && plan_of(g, kDftChunk, g->use_graphs).windows) || (rest > 1 && plan_of(g, rest, false).windows);
+}
+
 // Lays out the second copy of the state and 1/eps of a grid that takes its
 // steps in windows, again after any change to it. A grid whose second copy
 // does not fit in device memory keeps the launches per half step.
-int ensure_window64(fdtd_grid* g);
-
 int ensure_window(fdtd_grid* g) {
   if (g->win_version == g->version) return FDTD_OK;
   g->win_ok = false;
-  if (!window_wanted(g)) {
+  if (!g->win_wanted) {
     g->win_version = g->version;
     return FDTD_OK;
   }
@@ -1096,51 +1173,6 @@ int ensure_window64(fdtd_grid* g) {
   return FDTD_OK;
 }
 
-// Steps per launch and rows per window: the pair with the least modelled time
-// of a step. A launch takes from its predecessor's end about 4 us + 1.05 us a
-// step with windows of 32 rows, 8 us + 1.5 us a step with 64 (measured at
-// 317 x 233), and each further round of windows (two per SM) 5 and 11.5 us +
-// 0.1 us a step (3001 x 2047: 32 rows 19.7 us a step at 8 steps, 64 rows 20.9
-// at 4, 14.3 at 8, 14.2 at 12, 16.3 at 16).
-int window_steps(int nx, int ny, int* rows, int most_rows = kWinRows) {
-  int best = 8;
-  double least = 1e30;
-  for (int R : {32, 64})
-    if (R <= most_rows)
-    for (int L : {16, 12, 8, 6, 4}) {
-      const int T = (kGraphSteps + L - 1) / L;
-      if (4 * T > R + 16) continue;
-      const double rounds = window_count(nx, ny, R, T) / 296.0;
-      const double one = R == 32 ? 4.0 + 1.05 * T : 8.0 + 1.5 * T;
-      const double more = (R == 32 ? 5.0 : 11.5) + 0.1 * T;
-      const double t = (one + std::max(0.0, rounds - 1.0) * more) * L;
-      if (t < least) {
-        least = t;
-        best = T;
-        *rows = R;
-      }
-    }
-  return best;
-}
-
-// Steps per launch of FP64 windows, one per SM: a round of windows takes about
-// 10 us + 3 us a step (256 x 256: 21 us at 4 steps, 28 at 6, 33 at 8; 600 x 450
-// with poles and TFSF, two rounds at 5 and 6 steps: 57 and 63, three at 8: 116).
-int window64_steps(int nx, int ny) {
-  int best = 8;
-  double least = 1e30;
-  for (int L : {16, 14, 12, 10, 8, 6}) {
-    const int T = (kGraphSteps + L - 1) / L;
-    const double rounds = std::ceil(window64_count(nx, ny, T) / 148.0);
-    const double t = rounds * (10.0 + 3.0 * T) * L;
-    if (t < least) {
-      least = t;
-      best = T;
-    }
-  }
-  return best;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1189,8 +1221,9 @@ int fdtd_grid_create(const fdtd_grid_desc* desc, fdtd_grid** out) try {
       if (!rc && !g->f32) rc = dalloc(g, &g->B[c], fb);
     }
   }
+  cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, g->d.device);
   if (!rc) rc = dalloc(g, reinterpret_cast<void**>(&g->ctrl), sizeof(Control));
-  if (!rc) rc = dalloc(g, reinterpret_cast<void**>(&g->d_flag), sizeof(int));
+  if (!rc) rc = dalloc(g, reinterpret_cast<void**>(&g->d_flag), 4 * sizeof(int));
   if (!rc) {
     void* ptrs[6] = {g->E[0], g->E[1], g->E[2], g->H[0], g->H[1], g->H[2]};
     rc = upload_vec(g, reinterpret_cast<void**>(&g->d_fieldptrs), ptrs, sizeof(ptrs));
@@ -1297,6 +1330,7 @@ int fdtd_set_materials(fdtd_grid* g, const fdtd_material* mats, int n) try {
   }
   CK(cudaSetDevice(g->d.device));
   g->mats.assign(mats, mats + n);
+  g->material_version++;
   return build_materials(g);
 } catch (...) {
   return host_failure();
@@ -1310,6 +1344,7 @@ int fdtd_set_material_ids(fdtd_grid* g, const uint8_t* ids) try {
   uint8_t top = 0;
   for (long long c = 0; c < n; c++) top = ids[c] > top ? ids[c] : top;
   if (top >= g->mats.size()) return fail(FDTD_ERR_INVALID, "material id out of range of the material table");
+  g->material_version++;
   const size_t rows = static_cast<size_t>(g->n[1]) * g->n[2], rl = static_cast<size_t>(rowlen(g));
   CK(cudaSetDevice(g->d.device));
   if (g->d_bids) {
@@ -1344,6 +1379,7 @@ int fdtd_set_material_blocks(fdtd_grid* g, int block_shift, const uint16_t* ids,
     g->d_ids = nullptr;
   }
   g->bshift = block_shift;
+  g->material_version++;
   g->nbx = nbx;
   g->nby = nby;
   g->nbz = nbz;
@@ -1355,6 +1391,7 @@ int fdtd_set_material_blocks(fdtd_grid* g, int block_shift, const uint16_t* ids,
 int fdtd_set_eps_map(fdtd_grid* g, const double* eps) try {
   if (!g) return fail(FDTD_ERR_INVALID, "null grid");
   CK(cudaSetDevice(g->d.device));
+  g->material_version++;
   if (!eps) {
     if (g->d_eps_map) dfree(g, g->d_eps_map);
     g->d_eps_map = nullptr;
@@ -1697,7 +1734,8 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof);
 static void adjoint_capture_args(fdtd_adjoint* a, WinArgs& w);
 static int adjoint_capture_step(fdtd_adjoint* a, long long t, cudaStream_t s);
 static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof);
-static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoint* adj = nullptr);
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, bool graph, fdtd_adjoint* adj = nullptr);
+static int enqueue_run(fdtd_grid* g, int nsteps, cudaStream_t s, bool graph);
 
 // The TFSF aux tables for a call of nsteps steps: at least 257 rows, so that
 // calls of up to 256 steps keep them (and the step graph, whose launches hold
@@ -1726,7 +1764,7 @@ static int ensure_step_graph(fdtd_grid* g, cudaStream_t s) {
   }
   const long long before = g->launches;
   CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  int rc = g->win_ok ? enqueue_windows(g, kGraphSteps, s) : enqueue_steps(g, kGraphSteps, s, nullptr);
+  int rc = enqueue_run(g, kGraphSteps, s, true);
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &graph);
   if (rc) return rc;
@@ -1764,8 +1802,15 @@ int fdtd_prepare(fdtd_grid* g) try {
     rc = ensure_aux_tables(g, kGraphSteps);
     if (rc) return rc;
   }
-  rc = ensure_window(g);
+  rc = ensure_plans(g);
   if (rc) return rc;
+  // so that no later call lays out the windows
+  bool any = false;
+  for (int n = 2; n <= kDftChunk && !any; n++) any = takes_windows(g, n);
+  if (any) {
+    rc = ensure_window(g);
+    if (rc) return rc;
+  }
   if (graph) {
     if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
     rc = ensure_step_graph(g, g->stream);
@@ -1915,24 +1960,19 @@ static int enqueue_steps(fdtd_grid* g, int nsteps, cudaStream_t s, double* prof)
   return FDTD_OK;
 }
 
-// Enqueues nsteps steps of a grid that takes them in windows: an even number
-// of launches per stretch of steps (ending on the grid's own arrays), each
-// stretch within the DFT sample ring; a single step left over goes out as
-// launches per half step.
-// `adj`: the curl terms of the design cells of every step go to its store.
-static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoint* adj) {
+// Enqueues nsteps steps of a grid whose windows are laid out: each stretch of
+// steps within the DFT sample ring in an even number of launches (ending on the
+// grid's own arrays), or per half step where its plan says so; a single step left
+// over goes out as launches per half step.
+// `graph`: captured for a graph. `adj`: every stretch goes out in windows, and the
+// curl terms of the design cells of every step to its store.
+static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, bool graph, fdtd_adjoint* adj) {
   WinArgs wa = g->win;
   if (adj) adjoint_capture_args(adj, wa);
   const bool dft = !g->dfts.empty();
   bool ring = false;  // a region holds cells of the outer ring
   for (const auto& r : g->dfts)
     for (int d = 0; d < 2; d++) ring = ring || r.lo[d] == 0 || r.hi[d] == g->n[d] - 1;
-  int rows = kWinRows;
-  // with Lorentz poles a window of 64 rows is more than an SM's shared memory;
-  // with Drude poles one fits instead of two and is still the faster (3000 x
-  // 2000: 22.2 us a step against 25.5 in windows of 32 rows)
-  const int most = g->f32 && g->max_poles > 0 ? 32 : kWinRows;
-  const int T = g->f32 ? window_steps(g->n[0], g->n[1], &rows, most) : window64_steps(g->n[0], g->n[1]);
   PlainArgs pa;
   FusedArgs fa;
   const bool tfsf = !g->planes.empty();
@@ -1941,20 +1981,21 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
   const WinExt* const ext = g->f32 && (tfsf || g->max_poles != 0) ? &g->win_ext : nullptr;
   for (int done = 0; done < nsteps;) {
     const int n = std::min(nsteps - done, kDftChunk - (dft ? g->dft_pending : 0));
-    if (n == 1) {
+    const WindowPlan plan = n > 1 ? plan_of(g, n, graph) : WindowPlan{};
+    if (n == 1 || (!adj && !plan.windows)) {
       if (adj) g->launches += adjoint_capture_step(adj, done, s);
-      const int rc = enqueue_steps(g, 1, s, nullptr);
+      const int rc = enqueue_steps(g, n, s, nullptr);
       if (rc) return rc;
-      done++;
+      done += n;
       continue;
     }
-    const int L = 2 * ((n + 2 * T - 1) / (2 * T));
+    const int L = plan.launches;
     if (tfsf && g->f32) g->launches += launch_tfsf_fused_table(g->d.mode, fa, n, g->tfsf_cells, static_cast<float*>(g->win_tfsf), s);
     if (tfsf && !g->f32) g->launches += launch_tfsf_table(g->d.mode, pa, n, static_cast<double*>(g->win_tfsf), s);
     for (int q = 0; q < L; q++) {
       const int at = static_cast<int>(static_cast<long long>(n) * q / L);
       const int t = static_cast<int>(static_cast<long long>(n) * (q + 1) / L) - at;
-      g->launches += g->f32 ? launch_window(g->d.mode, wa, ext, rows, t, at, q & 1, g->dft_pending + at, s)
+      g->launches += g->f32 ? launch_window(g->d.mode, wa, ext, plan.rows, t, at, q & 1, g->dft_pending + at, s)
                             : launch_window64(g->d.mode, g->win64, t, at, q & 1, g->dft_pending + at, s);
     }
     if ((adj || ext) && ring) g->launches += launch_window_ring(g->d.mode, wa, g->dft_maxpts, g->dft_pending, n, s);
@@ -1968,6 +2009,10 @@ static int enqueue_windows(fdtd_grid* g, int nsteps, cudaStream_t s, fdtd_adjoin
   if (g->dft_pending > 0) g->launches += flush_dft(g, s);
   CK(cudaGetLastError());
   return FDTD_OK;
+}
+
+static int enqueue_run(fdtd_grid* g, int nsteps, cudaStream_t s, bool graph) {
+  return g->win_ok && g->win_version == g->version ? enqueue_windows(g, nsteps, s, graph) : enqueue_steps(g, nsteps, s, nullptr);
 }
 
 static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
@@ -1989,8 +2034,11 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     }
     prc = ensure_aux_tables(g, nsteps);
     if (prc) return prc;
-    prc = ensure_window(g);
-    if (prc) return prc;
+    if (nsteps > 1 && !prof) {
+      prc = ensure_plans(g);
+      if (!prc && takes_windows(g, nsteps)) prc = ensure_window(g);
+      if (prc) return prc;
+    }
   }
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
   if (s != g->stream) {
@@ -2024,7 +2072,7 @@ static int step_impl(fdtd_grid* g, int nsteps, void* stream, double* prof) {
     }
   }
   if (done < nsteps) {
-    int rc = g->win_ok && !prof ? enqueue_windows(g, nsteps - done, s) : enqueue_steps(g, nsteps - done, s, prof);
+    int rc = prof ? enqueue_steps(g, nsteps - done, s, prof) : enqueue_run(g, nsteps - done, s, false);
     if (rc) return rc;
   }
   CK(cudaGetLastError());
@@ -2230,6 +2278,15 @@ int fdtd_copy_plane_between(fdtd_grid* src, int which, int k_src, fdtd_grid* dst
 int fdtd_use_graphs(fdtd_grid* g, int enable) try {
   if (!g) return fail(FDTD_ERR_INVALID, "null grid");
   g->use_graphs = enable != 0;
+  return FDTD_OK;
+} catch (...) {
+  return host_failure();
+}
+
+int fdtd_always_window(fdtd_grid* g, int enable) try {
+  if (!g) return fail(FDTD_ERR_INVALID, "null grid");
+  g->win_always = enable != 0;
+  g->version++;
   return FDTD_OK;
 } catch (...) {
   return host_failure();
@@ -3378,6 +3435,7 @@ static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
   fdtd_grid* g = a->g;
   *done = false;
   int rc = ensure_pml(g);
+  if (!rc) rc = ensure_plans(g);
   if (!rc) rc = ensure_window(g);
   if (rc || !g->win_ok) return rc;
   size_t free_b = 0, total_b = 0;
@@ -3405,7 +3463,7 @@ static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
     return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
   }
   if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
-  rc = enqueue_windows(g, nsteps, g->stream, a);
+  rc = enqueue_windows(g, nsteps, g->stream, false, a);
   if (rc) return rc;
   g->t += nsteps;
   *done = true;
@@ -3447,7 +3505,7 @@ static int adj_backward_stored(fdtd_adjoint* a, const FusedArgs& fa) {
   w.grad = a->d_grad;
   g->launches += launch_adjoint_force(a->d_X, a->freq, np, static_cast<int>(a->nsteps), a->d_force, s);
   int rows = kWinRows, from = 0;
-  const int T = window_steps(g->n[0], g->n[1], &rows);
+  const int T = adjoint_window_steps(g->n[0], g->n[1], g->sms, &rows);
   for (int t = static_cast<int>(a->nsteps) - 1; t >= 0; t -= T) {
     g->launches += launch_adjoint_window(w, rows, std::min(T, t + 1), t, from, s);
     from = 1 - from;

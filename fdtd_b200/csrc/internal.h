@@ -277,7 +277,7 @@ struct DftRegionDev {
 
 // Temporal blocking of 2D FP32 grids (kernels_window.cu): windows of
 // kWinCols x 64 (or 32) cells take up to kWinMaxSteps steps per launch
-constexpr int kWinCols = 64, kWinRows = 64, kWinMaxSteps = 16;
+constexpr int kWinCols = 64, kWinRows = 64, kWin64Rows = 32, kWinMaxSteps = 16;
 constexpr int kWinMaxBoxes = 8, kWinMaxRegions = 32;
 
 struct WinBox {  // box source, E (target 0) or H (2)
@@ -352,6 +352,10 @@ inline int window_count(int nx, int ny, int rows, int T) {
 // counter; DFT samples go to ring slots slot .. slot + T - 1
 // (x: null, or what the grid's poles and TFSF planes need)
 int launch_window(int mode, const WinArgs& a, const WinExt* x, int rows, int T, int s, int from, int slot, cudaStream_t st);
+// counts[0] and [1]: the 64 x 32 and the 64 x 64 cell blocks of the grid that hold
+// cells with poles
+int launch_pole_blocks(const FusedArgs& a, unsigned* counts, cudaStream_t s);
+int launch_pole_blocks(const PlainArgs& a, unsigned* counts, cudaStream_t s);
 // the ring's samples of n steps in slots slot .. slot + n - 1, from the ring's
 // values (which it keeps), for windows that do not see to them themselves (a.cap, poles, planes)
 int launch_window_ring(int mode, const WinArgs& a, const long long (&max_pts)[2], int slot, int n, cudaStream_t s);
@@ -414,7 +418,9 @@ struct Win64Args {
 };
 // poles times E components that a window's shared memory holds P and J of
 constexpr int kWin64Poles = 2;
-int window64_count(int nx, int ny, int T);
+inline int window64_count(int nx, int ny, int T) {
+  return window_tiles(nx, kWinCols, kWinCols - 2 * T) * window_tiles(ny, kWin64Rows, kWin64Rows - 2 * T);
+}
 int launch_window64(int mode, const Win64Args& a, int T, int s, int from, int slot, cudaStream_t st);
 // the TFSF corrections of the nsteps steps from the counter on
 int launch_tfsf_table(int mode, const PlainArgs& a, int nsteps, double* out, cudaStream_t s);

@@ -951,6 +951,29 @@ __global__ void window_cells_kernel(const __grid_constant__ FusedArgs a, unsigne
   disp[c] = static_cast<unsigned short>(n == 0 ? 0 : (n < 0 ? 1 : n) << 14 | mid);
 }
 
+// A 64 x 64 cell block per CTA, its halves of 32 rows one after another
+__device__ __forceinline__ bool has_poles(const MatF32& m) { return m.npoles != 0; }
+__device__ __forceinline__ bool has_poles(const MatF64& m) { return m.kind >= 2; }
+template <class Args, class Mat>
+__global__ void __launch_bounds__(256) pole_blocks_kernel(const __grid_constant__ Args a, const Mat* mats, int pitch, unsigned* counts) {
+  int found[2];
+  for (int h = 0; h < 2; h++) {
+    int any = 0;
+    for (int q = threadIdx.x; q < 64 * 32; q += 256) {
+      const int i = blockIdx.x * 64 + q % 64, j = blockIdx.y * 64 + h * 32 + q / 64;
+      if (i >= a.nx || j >= a.ny) continue;
+      int mid = 0;
+      if (a.ids) mid = a.ids[static_cast<long long>(j) * pitch + i];
+      else if (a.bids) mid = a.bids[(j >> a.bshift) * a.nbx + (i >> a.bshift)];
+      any |= has_poles(mats[mid]);
+    }
+    found[h] = __syncthreads_or(any) != 0;
+  }
+  if (threadIdx.x != 0 || found[0] + found[1] == 0) return;
+  atomicAdd(counts, found[0] + found[1]);
+  atomicAdd(counts + 1, 1);
+}
+
 // the samples of the outer ring's cells in slots slot .. slot + n - 1, one region
 // per blockIdx.y, a thread per point
 __global__ void __launch_bounds__(256) window_ring_kernel(const __grid_constant__ WinArgs a, int mode, int h, int slot, int n) {
@@ -985,6 +1008,16 @@ void window_ext_go(F fn, int mode, int n, cudaStream_t st, const WinArgs& a, con
 
 int launch_window_cells(const FusedArgs& a, unsigned short* disp, cudaStream_t s) {
   window_cells_kernel<<<dim3((a.pitch + 31) / 32, (a.ny + 7) / 8), dim3(32, 8), 0, s>>>(a, disp);
+  return 1;
+}
+
+int launch_pole_blocks(const FusedArgs& a, unsigned* counts, cudaStream_t s) {
+  pole_blocks_kernel<<<dim3((a.nx + 63) / 64, (a.ny + 63) / 64), 256, 0, s>>>(a, a.mats, a.pitch, counts);
+  return 1;
+}
+
+int launch_pole_blocks(const PlainArgs& a, unsigned* counts, cudaStream_t s) {
+  pole_blocks_kernel<<<dim3((a.nx + 63) / 64, (a.ny + 63) / 64), 256, 0, s>>>(a, a.mats, a.nx, counts);
   return 1;
 }
 

@@ -26,7 +26,7 @@ namespace fdtdb {
 namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
-constexpr int kRows = 32;  // a warp per row
+constexpr int kRows = kWin64Rows;  // a warp per row
 constexpr int kCells = kWinCols * kRows;
 
 // what acts on cells of the window besides the update: a source (its values
@@ -615,10 +615,6 @@ void window64_go(const Win64Args& a, int n, int T, int s, int from, int slot, cu
 }
 
 }  // namespace
-
-int window64_count(int nx, int ny, int T) {
-  return window_tiles(nx, kWinCols, kWinCols - 2 * T) * window_tiles(ny, kRows, kRows - 2 * T);
-}
 
 int launch_window64(int mode, const Win64Args& a, int T, int s, int from, int slot, cudaStream_t st) {
   const int n = window64_count(a.nx, a.ny, T);

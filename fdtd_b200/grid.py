@@ -32,7 +32,7 @@ STATUS = {0: "FDTD_OK", -1: "FDTD_ERR_INVALID", -2: "FDTD_ERR_CUDA", -3: "FDTD_E
 # every symbol include/fdtd_b200.h declares
 EXPORTS = ["fdtd_grid_create", "fdtd_grid_destroy", "fdtd_set_pml", "fdtd_set_pml_model", "fdtd_set_materials", "fdtd_set_material_ids",
            "fdtd_set_material_blocks", "fdtd_set_eps_map", "fdtd_set_boundary", "fdtd_set_time_scheme", "fdtd_add_source", "fdtd_add_source_box", "fdtd_add_tfsf_plane", "fdtd_add_dft",
-           "fdtd_dft_npoints", "fdtd_dft_read", "fdtd_read_quantity", "fdtd_step", "fdtd_prepare", "fdtd_step_static_scratch", "fdtd_step_half", "fdtd_step_half_part", "fdtd_copy_plane", "fdtd_copy_plane_between", "fdtd_material_explicit", "fdtd_profile_step", "fdtd_set_sweep_kernel", "fdtd_use_graphs", "fdtd_error_flags", "fdtd_synchronize", "fdtd_download", "fdtd_upload",
+           "fdtd_dft_npoints", "fdtd_dft_read", "fdtd_read_quantity", "fdtd_step", "fdtd_prepare", "fdtd_step_static_scratch", "fdtd_step_half", "fdtd_step_half_part", "fdtd_copy_plane", "fdtd_copy_plane_between", "fdtd_material_explicit", "fdtd_profile_step", "fdtd_set_sweep_kernel", "fdtd_use_graphs", "fdtd_always_window", "fdtd_error_flags", "fdtd_synchronize", "fdtd_download", "fdtd_upload",
            "fdtd_check_finite", "fdtd_field_error", "fdtd_get_step", "fdtd_launch_count", "fdtd_memory_bytes",
            "fdtd_batch_create", "fdtd_batch_destroy", "fdtd_batch_tune", "fdtd_batch_configure", "fdtd_batch_step",
            "fdtd_batch_info", "fdtd_batch_item_rows", "fdtd_batch_set_item_rows", "fdtd_batch_set_temporal",
@@ -100,6 +100,7 @@ def load_library(path: str = LIB_PATH):
         "fdtd_profile_step": [vp, i, vp, dp],
         "fdtd_set_sweep_kernel": [vp, i],
         "fdtd_use_graphs": [vp, i],
+        "fdtd_always_window": [vp, i],
         "fdtd_error_flags": [vp, ip],
         "fdtd_synchronize": [vp],
         "fdtd_download": [vp, i, dp],
@@ -328,6 +329,11 @@ class Grid:
 
     def use_graphs(self, enable: bool) -> None:
         _check(load_library().fdtd_use_graphs(self.h, 1 if enable else 0))
+
+    def always_window(self, enable: bool = True) -> None:
+        """2D grids: take steps in windows wherever these can hold the grid, not
+        only where they are the faster (fdtd_always_window)."""
+        _check(load_library().fdtd_always_window(self.h, 1 if enable else 0))
 
     def error_flags(self) -> int:
         v = ctypes.c_int()

@@ -214,12 +214,13 @@ int fdtd_dft_read(fdtd_grid* g, int handle, double* out);
 /* Advance nsteps full time steps on `stream` (a cudaStream_t, or NULL for the
  * handle's stream). Returns once the work is enqueued. */
 int fdtd_step(fdtd_grid* g, int nsteps, void* stream);
-/* 2D grids take calls of two steps or more in windows: several steps per
- * launch, from one copy of the state into another (the grid holds a second
- * copy of what a step changes, and per-cell material factors). FP32 grids do
- * without mu_r != 1; FP64 grids with one mu_r, BD1, at most one pole (TE) or
- * two (TM) and 32 of sources, boxes and twice the TFSF planes; both without
- * boundary conditions and DFT of surface quantities.
+/* 2D grids take stretches of two steps or more in windows where that is the
+ * faster by a model fitted to measurements: several steps per launch, from one
+ * copy of the state into another (a grid that does holds a second copy of what
+ * a step changes, and per-cell material factors). FP32 grids may without
+ * mu_r != 1; FP64 grids with one mu_r, BD1, at most one pole (TE) or two (TM)
+ * and 32 of sources, boxes and twice the TFSF planes; both without boundary
+ * conditions and DFT of surface quantities.
  * Results are those of one launch per half step, which
  * fdtd_set_sweep_kernel(g, FDTD_SWEEP_REGS) brings back, and which a grid
  * keeps whose second copy finds no device memory. */
@@ -316,6 +317,9 @@ int fdtd_set_sweep_kernel(fdtd_grid* g, int kind);
 /* Replay a captured CUDA graph per 64 steps inside fdtd_step (default 1), or
  * launch every kernel from the host (0). Results are identical. */
 int fdtd_use_graphs(fdtd_grid* g, int enable);
+/* 2D grids: windows (see fdtd_step) wherever they can hold the grid (1), or where
+ * they are the faster (0, the default). Results are identical. */
+int fdtd_always_window(fdtd_grid* g, int enable);
 /* Device-side error flags accumulated by the kernels (0 = none; bit 0: a
  * bounded wait on a TMA stage expired and the sweep was abandoned; bit 1: in
  * the one-launch step an H tile's bounded wait for the E tiles it reads
