@@ -940,6 +940,11 @@ int ensure_plans(fdtd_grid* g) {
   if (g->plan_version == g->version) return FDTD_OK;
   g->win_wanted = window_wanted(g);
   g->plans.clear();
+  if (!g->win_wanted && g->win_block) {
+    dfree(g, g->win_block);
+    g->win_block = nullptr;
+    g->win_ok = false;
+  }
   if (g->win_wanted) {
     const int rc = ensure_pole_share(g);
     if (rc) return rc;
