@@ -224,6 +224,9 @@ struct fdtd_grid {
   WinArgs win{};
   Win64Args win64{};
   void* win_tfsf = nullptr;  // the TFSF corrections of a stretch of steps
+  // where the cells' factors lie in the block, and the materials they are of
+  void* win_factors[2]{};
+  long long win_materials = -1;
   WinExt win_ext;            // FP32: what poles and TFSF planes need
   long long win_version = -1;
   bool win_ok = false;
@@ -984,6 +987,35 @@ bool takes_windows(fdtd_grid* g, int nsteps) {
   return (nsteps >= kDftChunk && plan_of(g, kDftChunk, g->use_graphs).windows) || (rest > 1 && plan_of(g, rest, false).windows);
 }
 
+// The block of a grid's windows, `total` bytes; *ok false where it does not fit
+int window_block(fdtd_grid* g, size_t total, bool* ok) {
+  *ok = true;
+  if (g->win_block && g->sizes[g->win_block] == total) return FDTD_OK;
+  dfree(g, g->win_block);
+  g->win_materials = -1;
+  const int rc = dalloc(g, &g->win_block, total);
+  if (!rc) return FDTD_OK;
+  *ok = false;
+  g->win_version = g->version;
+  return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
+}
+
+// Fills the cells' factors a and b of the windows where they are not those of the
+// grid's materials. Windows on a stream of the caller's may still read the old
+// ones; those to come read them before they wait for the launch ahead of them
+// (launch_chained): all is in place once this returns.
+template <class Fill>
+int window_factors(fdtd_grid* g, void* a, void* b, Fill fill) {
+  if (g->win_materials == g->material_version && g->win_factors[0] == a && g->win_factors[1] == b) return FDTD_OK;
+  CK(cudaDeviceSynchronize());
+  g->launches += fill();
+  CK(cudaStreamSynchronize(g->stream));
+  g->win_factors[0] = a;
+  g->win_factors[1] = b;
+  g->win_materials = g->material_version;
+  return FDTD_OK;
+}
+
 // Lays out the second copy of the state and 1/eps of a grid that takes its
 // steps in windows, again after any change to it. A grid whose second copy
 // does not fit in device memory keeps the launches per half step.
@@ -1023,14 +1055,9 @@ int ensure_window(fdtd_grid* g) {
   for (auto* p : pj) extra(g->sizes[p]);
   extra(np > 0 ? static_cast<size_t>(field_elems(g)) * sizeof(unsigned short) : 0);
   extra(static_cast<size_t>(g->tfsf_cells) * 2 * kDftChunk * sizeof(float));
-  if (!g->win_block || g->sizes[g->win_block] != total) {
-    dfree(g, g->win_block);
-    const int rc = dalloc(g, &g->win_block, total);
-    if (rc) {
-      g->win_version = g->version;
-      return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
-    }
-  }
+  bool fits = false;
+  const int rc = window_block(g, total, &fits);
+  if (rc || !fits) return rc;
   g->win = window_args(g);
   char* const b = static_cast<char*>(g->win_block);
   for (int q = 0; q < 3; q++) g->win.f[1][q] = reinterpret_cast<float*>(b + at[q]);
@@ -1040,7 +1067,6 @@ int ensure_window(fdtd_grid* g) {
   if (!window_uniform(g)) {
     float* const ie = reinterpret_cast<float*>(b + at[8]);
     g->win.ie = ie;
-    g->launches += launch_adjoint_inv_eps(fused_args(g), ie, g->stream);
   }
   const FusedArgs fa = fused_args(g);
   WinExt& x = g->win_ext;
@@ -1052,7 +1078,6 @@ int ensure_window(fdtd_grid* g) {
     x.pj[1][q] = reinterpret_cast<float*>(b + more[q]);
   }
   unsigned short* const disp = reinterpret_cast<unsigned short*>(b + more[pj.size()]);
-  if (np > 0) g->launches += launch_window_cells(fa, disp, g->stream);
   x.disp = disp;
   x.mats = fa.mats;
   x.nplanes = fa.nplanes;
@@ -1063,9 +1088,11 @@ int ensure_window(fdtd_grid* g) {
   g->win_tfsf = b + more[pj.size() + 1];
   x.tfsf = static_cast<const float*>(g->win_tfsf);
   x.tfsf_cells = g->tfsf_cells;
-  // the windows read what was set up here before they wait for the launch
-  // ahead of them (launch_chained): it is all in place once this returns
-  CK(cudaStreamSynchronize(g->stream));
+  float* const ie = const_cast<float*>(g->win.ie);
+  const int frc = window_factors(g, ie, np > 0 ? disp : nullptr, [&] {
+    return (ie ? launch_adjoint_inv_eps(fa, ie, g->stream) : 0) + (np > 0 ? launch_window_cells(fa, disp, g->stream) : 0);
+  });
+  if (frc) return frc;
   g->win_version = g->version;
   g->win_ok = true;
   return FDTD_OK;
@@ -1104,14 +1131,9 @@ int ensure_window64(fdtd_grid* g) {
   part(window_uniform(g) ? 0 : cells * sizeof(double));
   part(np > 0 ? cells * sizeof(unsigned short) : 0);
   part(static_cast<size_t>(g->tfsf_cells) * 3 * 2 * kDftChunk * sizeof(double));
-  if (!g->win_block || g->sizes[g->win_block] != total) {
-    dfree(g, g->win_block);
-    const int rc = dalloc(g, &g->win_block, total);
-    if (rc) {
-      g->win_version = g->version;
-      return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
-    }
-  }
+  bool fits = false;
+  const int rc = window_block(g, total, &fits);
+  if (rc || !fits) return rc;
   char* const b = static_cast<char*>(g->win_block);
   auto twin = [&](size_t q) { return own[q] ? reinterpret_cast<double*>(b + at[q]) : nullptr; };
   const PlainArgs pa = plain_args(g);
@@ -1155,7 +1177,6 @@ int ensure_window64(fdtd_grid* g) {
   w.disp = disp;
   w.np = np;
   w.mats = pa.mats;
-  if (den || disp) g->launches += launch_window64_cells(pa, den, disp, g->stream);
   w.nsrc = wa.nsrc;
   w.nbox = wa.nbox;
   w.nplanes = pa.nplanes;
@@ -1172,7 +1193,8 @@ int ensure_window64(fdtd_grid* g) {
     w.dft_pts[ph] = g->dft_pts[ph];
   }
   w.ctrl = g->ctrl;
-  CK(cudaStreamSynchronize(g->stream));  // as for the FP32 windows
+  const int frc = window_factors(g, den, disp, [&] { return den || disp ? launch_window64_cells(pa, den, disp, g->stream) : 0; });
+  if (frc) return frc;
   g->win_version = g->version;
   g->win_ok = true;
   return FDTD_OK;
