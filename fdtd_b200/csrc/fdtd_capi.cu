@@ -2690,8 +2690,9 @@ void tb_release(fdtd_batch* b) {
 
 // The second copy of every array a step changes (fields, CPML integrators,
 // the soft sources' last values), 1/eps per cell and the windows' arguments;
-// laid out once. On failure nothing is kept.
-int tb_prepare(fdtd_batch* b) {
+// laid out once. On failure nothing is kept; *no_memory says whether it was for
+// want of device memory.
+int tb_prepare(fdtd_batch* b, bool* no_memory = nullptr) {
   if (b->d_win) return FDTD_OK;
   CK(cudaDeviceSynchronize());
   std::vector<WinArgs> args;
@@ -2725,6 +2726,7 @@ int tb_prepare(fdtd_batch* b) {
   if (!ok) {
     const cudaError_t e = cudaGetLastError();
     tb_release(b);
+    if (no_memory) *no_memory = e == cudaErrorMemoryAllocation;
     return fail(FDTD_ERR_CUDA, std::string("temporal blocking: the second copy of the state: ") + cudaGetErrorString(e));
   }
   return FDTD_OK;
@@ -2992,9 +2994,12 @@ int fdtd_batch_tune(fdtd_batch* b, int steps) try {
   int best_tb = 0;
   b->tb_ms.assign(3, 0.f);
   if (!rc && !tb_unsupported(b)) {
-    rc = tb_prepare(b);
+    // a second copy that does not fit is one mode less, no failure
+    bool no_memory = false;
+    rc = tb_prepare(b, &no_memory);
+    if (no_memory) rc = FDTD_OK;
     if (!rc) rc = batch_items(b, best_rows);
-    for (int depth = 2; depth <= 4 && !rc; depth++) {
+    for (int depth = 2; depth <= 4 && !rc && b->d_win; depth++) {
       const int n = (steps + 4 * depth - 1) / (4 * depth) * (4 * depth);
       b->tb = depth;
       rc = tb_ready(b, n);
