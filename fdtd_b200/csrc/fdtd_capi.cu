@@ -322,6 +322,15 @@ void dfree(fdtd_grid* g, void* p) {
   cudaFree(p);
 }
 
+// Copies host memory to the device, in place for the work of every stream once
+// this returns. (From pageable memory cudaMemcpy returns once the data are
+// staged, and a small copy may wait its turn behind work of other streams; the
+// grids' and batches' streams do not wait for the stream it goes by.)
+cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 int upload_vec(fdtd_grid* g, void** p, const void* src, size_t bytes) {
   if (*p) dfree(g, *p);
   int rc = dalloc(g, p, bytes);
@@ -2490,7 +2499,7 @@ int fdtd_upload(fdtd_grid* g, int which, const double* host) try {
         if (g->f32) reinterpret_cast<float*>(buf.data())[q] = static_cast<float>(v);
         else reinterpret_cast<double*>(buf.data())[q] = v;
       }
-  CK(cudaMemcpy(p, buf.data(), buf.size(), cudaMemcpyHostToDevice));
+  CK(copy_in(p, buf.data(), buf.size()));
   return FDTD_OK;
 } catch (...) {
   return host_failure();
@@ -2648,13 +2657,13 @@ int batch_items(fdtd_batch* b, int rows) {
     const int tx = g->pitch / 128, ty = (g->n[1] - 2 + R - 1) / R;
     for (int t = 0; t < tx * ty; t++) items.push_back(static_cast<unsigned>(q) << 24 | static_cast<unsigned>(t));
   }
-  CK(cudaMemcpy(b->d_args, b->h_args.data(), b->h_args.size() * sizeof(FusedArgs), cudaMemcpyHostToDevice));
+  CK(copy_in(b->d_args, b->h_args.data(), b->h_args.size() * sizeof(FusedArgs)));
   // consecutive items (tiles of one grid) go to consecutive CTAs
   b->nitems = static_cast<int>(items.size());
   if (b->d_items) cudaFree(b->d_items);
   b->d_items = nullptr;
   CK(cudaMalloc(&b->d_items, items.size() * sizeof(unsigned)));
-  CK(cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+  CK(copy_in(b->d_items, items.data(), items.size() * sizeof(unsigned)));
   void* fn = batch_kernel_ptr(b->mode, b->maxp, rows);
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * rows, 0));
@@ -2721,7 +2730,7 @@ int tb_prepare(fdtd_batch* b, bool* no_memory = nullptr) {
     args.push_back(a);
   }
   if (ok) ok = cudaMalloc(&b->d_win, args.size() * sizeof(WinArgs)) == cudaSuccess;
-  if (ok) ok = cudaMemcpy(b->d_win, args.data(), args.size() * sizeof(WinArgs), cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) ok = copy_in(b->d_win, args.data(), args.size() * sizeof(WinArgs)) == cudaSuccess;
   if (ok) ok = cudaDeviceSynchronize() == cudaSuccess;
   if (!ok) {
     const cudaError_t e = cudaGetLastError();
@@ -2744,8 +2753,10 @@ int tb_windows(fdtd_batch* b, int T) {
   }
   unsigned* d = nullptr;
   CK(cudaMalloc(&d, items.size() * sizeof(unsigned)));
+  const cudaError_t e = copy_in(d, items.data(), items.size() * sizeof(unsigned));
+  if (e != cudaSuccess) cudaFree(d);
+  CK(e);
   b->tb_items[T] = {d, static_cast<int>(items.size())};
-  CK(cudaMemcpy(d, items.data(), items.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
   return FDTD_OK;
 }
 
@@ -2860,7 +2871,7 @@ int fdtd_batch_create(int n, fdtd_grid* const* grids, fdtd_batch** out) try {
     ctrls.push_back(g->ctrl);
   }
   CK(cudaMalloc(&b->d_args, args.size() * sizeof(FusedArgs)));
-  CK(cudaMemcpy(b->d_args, args.data(), args.size() * sizeof(FusedArgs), cudaMemcpyHostToDevice));
+  CK(copy_in(b->d_args, args.data(), args.size() * sizeof(FusedArgs)));
   b->h_args = args;
   b->mult.assign(b->grids.size(), 1);
   {
@@ -2874,9 +2885,12 @@ int fdtd_batch_create(int n, fdtd_grid* const* grids, fdtd_batch** out) try {
     for (size_t r = 0; r < order.size(); r++) b->cls[order[r]] = static_cast<int>(r * nc / order.size());
   }
   CK(cudaMalloc(&b->d_ctrls, ctrls.size() * sizeof(Control*)));
-  CK(cudaMemcpy(b->d_ctrls, ctrls.data(), ctrls.size() * sizeof(Control*), cudaMemcpyHostToDevice));
+  CK(copy_in(b->d_ctrls, ctrls.data(), ctrls.size() * sizeof(Control*)));
   CK(cudaMalloc(&b->d_ctl, sizeof(BatchCtl)));
-  CK(cudaMemset(b->d_ctl, 0, sizeof(BatchCtl)));
+  {
+    const BatchCtl zero{};
+    CK(copy_in(b->d_ctl, &zero, sizeof(zero)));
+  }
   int rc = batch_items(b, 4);
   if (rc) {
     fdtd_batch_destroy(b);
