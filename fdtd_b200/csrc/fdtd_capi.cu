@@ -2150,6 +2150,11 @@ static int half_step_impl(fdtd_grid* g, int phase, int part, void* stream) {
     return fail(FDTD_ERR_UNSUPPORTED, "a half step splits along z on 3D grids of 2 or more interior planes");
   CK(cudaSetDevice(g->d.device));
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
+  {
+    // lays the CPML out by the grid's own stream, which the caller's waits for next
+    const int prc = ensure_pml(g);
+    if (prc) return prc;
+  }
   if (s != g->stream && part != 1) CK(cudaStreamSynchronize(g->stream));
   if (part != 1 && g->dirty_dft) {
     int rc = rebuild_dft(g);
@@ -2173,10 +2178,6 @@ static int half_step_impl(fdtd_grid* g, int phase, int part, void* stream) {
                                            a.d_tab, a.d_tab + a.cap * L, s);
     }
     if (!g->auxes.empty()) g->launches += launch_chunk_start(g->ctrl, s);
-  }
-  {
-    const int prc = ensure_pml(g);
-    if (prc) return prc;
   }
   FusedArgs fa;
   PlainArgs pa;
