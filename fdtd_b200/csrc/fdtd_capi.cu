@@ -3509,6 +3509,8 @@ static int adj_forward_stored(fdtd_adjoint* a, int nsteps, bool* done) {
     adj_release(a);
     return rc == FDTD_ERR_NOMEM ? FDTD_OK : rc;
   }
+  // (a row's values beyond its last cell are read in pairs with it, and stay)
+  CK(cudaMemsetAsync(a->d_ie, 0, fe * sizeof(float), g->stream));
   if (g->dft_pending > 0) g->launches += flush_dft(g, g->stream);
   rc = enqueue_windows(g, nsteps, g->stream, false, a);
   if (rc) return rc;
