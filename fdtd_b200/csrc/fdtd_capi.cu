@@ -3219,7 +3219,8 @@ int fdtd_batch_error_flags(fdtd_batch* b, int* flags) try {
 // cudaMalloc when a call asks for more steps than any call before. Here the
 // table lives in the fixed array below instead, so stepping allocates nothing:
 // no cudaMalloc, no cudaFree, no allocating library call, no graph. Steps run
-// as eagerly launched kernels, the same kernels and order as fdtd_step.
+// as eagerly launched kernels per half step, on 2D grids too, whose windows in
+// fdtd_step need a second copy of the state; the results are the same.
 //
 // * Size limit: kStaticAuxBytes (4 MiB) for the tables of all planes of one
 //   call, i.e. at most 4 MiB / (16 bytes x sum of the planes' L) - 1 steps per
@@ -3348,13 +3349,21 @@ extern "C" int fdtd_step_static_scratch(fdtd_grid* g, int nsteps, void* stream) 
 // Adjoint gradient d(objective)/d(eps_r) of a 2D TM FP32 fused grid.
 //
 // Objective: J = sum over a probe box of |X|^2, X the running DFT of Ez at
-// one frequency. Forward: the grid's own steps (graph-replayed), with a copy
-// of the whole time-stepped state (E, H, CPML integrators, source history,
-// step counter) every `ckpt_every` steps. Backward, per checkpoint segment
-// from the last: restore the checkpoint, recompute the segment's steps with
-// the same kernels (no DFT), keeping d_t of each design cell, then reverse
-// the segment's steps with the adjoint kernels of kernels_adjoint.cu. At the
-// end the grid is put back to its state after the forward.
+// one frequency. The gradient sums the adjoint state times d_t, the curl term
+// of each design cell at each step t. Two forms, equal value for value:
+//
+// With kept terms (adj_forward_stored says where): the forward takes its steps
+// in windows and writes every d_t on the way; the backward reverses several
+// steps per launch (adjoint_window_kernel) and leaves the grid alone.
+//
+// With checkpoints, for the other grids. Forward: the grid's own steps
+// (graph-replayed), with a copy of the whole time-stepped state (E, H, CPML
+// integrators, source history, step counter) every `ckpt_every` steps.
+// Backward, per checkpoint segment from the last: restore the checkpoint,
+// recompute the segment's steps with the same kernels (no DFT), keeping d_t of
+// each design cell, then reverse the segment's steps with the adjoint kernels
+// of kernels_adjoint.cu. At the end the grid is put back to its state after the
+// forward.
 namespace {
 
 struct AdjBuf {

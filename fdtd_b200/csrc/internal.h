@@ -316,8 +316,6 @@ struct alignas(16) WinArgs {
   int dlo[2], dhi[2];
 };
 
-// windows along an axis of n cells, each w cells wide, o of them its own
-// (the first and the last own their cells up to the axis' end)
 // What the windows of a grid with poles or TFSF planes take besides.
 struct WinPlane {
   int axis, lo[2], hi[2];
@@ -343,6 +341,8 @@ __device__ __forceinline__ float lorentz_current(float a, float j, float b, floa
   return __fmaf_rn(-c, p, drude_current(a, j, b, e));
 }
 
+// windows along an axis of n cells, each w cells wide, o of them its own
+// (the first and the last own their cells up to the axis' end)
 __host__ __device__ inline int window_tiles(int n, int w, int o) { return n <= w ? 1 : 1 + (n - w + o - 1) / o; }
 // windows of `rows` rows of an nx x ny grid taking T steps
 inline int window_count(int nx, int ny, int rows, int T) {

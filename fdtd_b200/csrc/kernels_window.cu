@@ -3,8 +3,9 @@
 // A small 2D grid's step is a chain of launches that each last as long as a
 // few dependent L2 round trips; a large one moves its whole state through
 // memory twice per step. Both costs are per launch, so one launch here takes
-// T steps. A CTA holds a window of 64 x (4 NW) cells of one grid in registers
-// (each lane two neighbouring columns, each of its NW warps four rows),
+// T steps. A CTA holds a window of 64 x (R NW) cells of one grid in registers
+// (each lane two neighbouring columns, each of its NW warps R rows: 64 rows in
+// all with R = 4, 32 with R = 2),
 // advances it T steps and writes back the inner cells that T steps leave
 // exact: a step's dependence reaches one cell each way (E from H at i-1, j-1;
 // H from E at i+1, j+1), so values within T cells of a window edge inside the

@@ -309,7 +309,7 @@ class Grid:
         _check(load_library().fdtd_material_explicit(self.h, int(ft), ctypes.c_void_p(stream) if stream else None))
 
     def step_static_scratch(self, n: int, stream: Optional[int] = None) -> None:
-        """step() that allocates no device memory: the TFSF table of the call
+        """step() by launches per half step that allocates no device memory: the TFSF table of the call
         lives in a fixed 4 MiB device array shared by all grids of the device
         (at most 4 MiB / (16 B x sum of the planes' aux lengths) - 1 steps per
         call; calls that overlap on the GPU race on the array)."""
@@ -317,7 +317,8 @@ class Grid:
 
     def profile_step(self, n: int, stream: Optional[int] = None) -> dict:
         """Mean per-step kernel times (ms) over n steps, from CUDA events
-        recorded around each kernel on its launching stream."""
+        recorded around each kernel on its launching stream: the launches per
+        half step, on 2D grids too, which step() may advance in windows."""
         ms = np.zeros(5, dtype=np.float64)
         _check(load_library().fdtd_profile_step(self.h, int(n), ctypes.c_void_p(stream) if stream else None, _dp(ms)))
         return dict(zip(["e_sweep", "e_extra", "h_sweep", "h_extra", "advance_flush"], ms.tolist()))

@@ -275,8 +275,9 @@ int fdtd_material_explicit(fdtd_grid* g, int ft, void* stream);
  * from construction). */
 int fdtd_prepare(fdtd_grid* g);
 /* fdtd_step for callers that cannot allocate device memory while stepping
- * (no counterpart in the reference, whose steps run on the host). Same
- * kernels, order and results as fdtd_step, launched eagerly; the per-call
+ * (no counterpart in the reference, whose steps run on the host). The results
+ * of fdtd_step, by launches per half step (2D grids too, which take no windows
+ * here), launched eagerly; the per-call
  * TFSF incident-field table goes into one fixed 4 MiB device array instead of
  * a buffer that grows with cudaMalloc, so a call allocates nothing.
  * - At most 4 MiB / (16 bytes x the sum of the planes' aux lengths L) - 1
@@ -298,7 +299,9 @@ int fdtd_step_static_scratch(fdtd_grid* g, int nsteps, void* stream);
  * step: ms[0..4] receive the mean per-step time (milliseconds) of the E sweep,
  * the E-phase extras (TFSF kernel of the FP32 method, DFT gather), the H sweep,
  * the H-phase extras, and the step counter plus the amortised DFT flush.
- * Synchronises after every step; for measurement, not production. */
+ * Times the launches per half step, with the results of fdtd_step: 2D grids
+ * that fdtd_step advances in windows of several steps per launch spend other
+ * times there. Synchronises after every step; for measurement, not production. */
 int fdtd_profile_step(fdtd_grid* g, int nsteps, void* stream, double* ms);
 /* Which kernels carry the 3D FP32 fused sweeps: FDTD_SWEEP_AUTO (the
  * default: currently the staged sweeps, the fastest measured on B200), FDTD_SWEEP_REGS (z-marching, register prefetch),
