@@ -132,6 +132,10 @@ inline WindowPlan window_plan(const WindowCase& c, int n) {
   // (windows where the two come out alike: over 6156 measured calls the choice is
   // 0.3% slower than the better of the two, and more than 4% slower in 2.5%)
   best.windows = best.launches > 0 && best.us <= 1.03 * best.half_us;
+  // FP64 windows of one step move the state as often as the sweeps do, and their
+  // halo besides: they gain by the planes, samples and boxes alone (the model has
+  // no term for it: 499 x 1917, 2 steps 88 us per half step and 92 in windows)
+  if (!c.f32 && n == 2 && c.planes + c.gathers + c.boxes == 0) best.windows = false;
   return best;
 }
 

@@ -38,6 +38,7 @@ const Measured kMeasured[] = {
     {false, true, 256, 256, 0, 0.000, 0.000, 0, 1, 64, 233, 472},
     {false, false, 256, 256, 0, 0.000, 0.000, 4, 0, 64, 388, 684},
     {false, false, 480, 700, 0, 0.000, 0.000, 0, 0, 2, 43, 34},
+    {false, false, 499, 1917, 0, 0.000, 0.000, 0, 0, 2, 92, 88},
     {false, true, 1200, 300, 0, 0.000, 0.000, 0, 0, 2, 43, 35},
     {false, false, 2000, 2000, 1, 0.100, 0.103, 4, 1, 16, 1227, 3154},
     {false, false, 2500, 2500, 1, 0.095, 0.098, 4, 1, 2, 547, 637},
