@@ -3060,7 +3060,7 @@ int fdtd_batch_set_temporal(fdtd_batch* b, int depth) try {
   if (depth != 0 && depth != 2 && depth != 3 && depth != 4)
     return fail(FDTD_ERR_INVALID, "temporal blocking depth must be 0, 2, 3 or 4");
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
+  CK(cudaDeviceSynchronize());  // steps on a stream of the caller's too
   if (depth > 0) {
     if (const char* why = tb_unsupported(b)) return fail(FDTD_ERR_UNSUPPORTED, why);
     const int rc = tb_prepare(b);
@@ -3089,7 +3089,7 @@ int fdtd_batch_configure(fdtd_batch* b, int persistent, int rows) try {
   if (!b) return fail(FDTD_ERR_INVALID, "null batch");
   if (rows != 1 && rows != 2 && rows != 4 && rows != 8) return fail(FDTD_ERR_INVALID, "rows must be 1, 2, 4 or 8");
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
+  CK(cudaDeviceSynchronize());  // steps on a stream of the caller's too
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->graphs.clear();
   tb_release(b);
@@ -3110,7 +3110,7 @@ int fdtd_batch_set_item_rows(fdtd_batch* b, const int* rows_per_grid) try {
     m[q] = r / b->rows;
   }
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
+  CK(cudaDeviceSynchronize());  // steps on a stream of the caller's too
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->graphs.clear();
   b->mult = m;

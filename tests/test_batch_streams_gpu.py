@@ -69,3 +69,28 @@ def test_first_calls_behind_another_batch(fdtd, mode, depth):
                 g.close()
     for a, c in zip(*out):
         assert np.array_equal(a, c) and np.any(a)
+
+
+@pytest.mark.parametrize("change", [lambda b: b.set_item_rows([4 * (1 + q % 2) for q in range(len(b.grids))]), lambda b: b.configure(False, 8),
+                                    lambda b: b.set_temporal(3)], ids=["item_rows", "configure", "temporal"])
+def test_set_up_behind_steps_on_a_caller_stream(fdtd, change):
+    """The launch mode of a batch set while its steps are in flight on a stream of
+    the caller's: the lists and arguments that those read stay until they are done."""
+    import torch
+    s = torch.cuda.Stream()
+    out = []
+    for wait in (True, False):
+        b = _batch(fdtd, P.TE, 12, 3, None)
+        b.step(150, stream=s.cuda_stream)
+        if wait:
+            s.synchronize()
+        change(b)
+        b.step(50, stream=s.cuda_stream)
+        s.synchronize()
+        out.append(_fields(b, P.TE))
+        grids = b.grids
+        b.close()
+        for g in grids:
+            g.close()
+    for a, c in zip(*out):
+        assert np.array_equal(a, c) and np.any(a)
