@@ -45,10 +45,27 @@ __device__ __forceinline__ void after_previous_launch() { asm volatile("griddepc
 constexpr unsigned long long kChainCtas = 16384;
 // whether a launch of this many CTAs is chained: one of many rounds of CTAs
 // gains nothing worth their waits
-inline bool chains(dim3 grid) { return static_cast<unsigned long long>(grid.x) * grid.y * grid.z <= kChainCtas; }
+inline unsigned long long ctas_of(dim3 grid) { return static_cast<unsigned long long>(grid.x) * grid.y * grid.z; }
+inline bool chains(dim3 grid) { return ctas_of(grid) <= kChainCtas; }
 
+// Launched one by one a chained kernel also hides its launch. Replayed from a graph
+// there is little to hide, and the sweeps, gathers and corrections of small 3D grids
+// lost by the chain; each has a rule of its own for launches under capture.
+inline bool under_capture(cudaStream_t s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
+}
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 148;
+}
+
+// chain: whether it is (its kernel waits all the same, which is free where it is not)
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+inline cudaError_t launch_chained_if(bool chain, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -58,8 +75,12 @@ inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = chains(grid) ? 1 : 0;
+  cfg.numAttrs = chain ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  return launch_chained_if(chains(grid), fn, grid, block, smem, s, args...);
 }
 
 // include/FDTDConstants.hpp:394-398
@@ -201,6 +222,7 @@ struct PlainArgs {
   const double* eps_map;  // per-cell relative permittivity of non-dispersive cells (> 0), or null
   int dispersive;      // most poles of any material (Drude: 1)
   int all_dispersive;  // every material has poles: P and J are read with the fields
+  int gathers;         // half steps with DFT regions to gather
   int single_mat;      // the table holds one material: no cell's id is read
   int uniform_mu;      // every material has the same mu_r: the H half reads no id
   int nsrc;

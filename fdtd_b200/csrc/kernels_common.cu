@@ -225,9 +225,13 @@ int launch_dft_gather(int precision, const DftRegionDev* regions, int nreg, long
     dft_gather_kernel<double><<<grid, 256, 0, s>>>(regions, total_pts, reinterpret_cast<const double* const*>(fields), ny,
                                                    pitch, static_cast<long long>(slot), static_cast<double*>(buf));
   else
-    launch_chained(dft_gather_kernel<float>, grid, dim3(256), 0, s, regions, total_pts,
-                   reinterpret_cast<const float* const*>(fields), ny, pitch, static_cast<long long>(slot),
-                   static_cast<float*>(buf));
+    // FP32 ones are where they are small: faces of a box, us a step chained and not:
+    // in a graph 60 CTAs (132 x 64 x 60) 29.6 and 30.1, 120 (98 x 150 x 45) 35.4 and
+    // 33.5, 228 (173 x 150 x 141) 94.0 and 84.5; launched one by one 132 CTAs (128 x
+    // 128 x 64) 39.7 and 41.3, 228 97.1 and 92.1
+    launch_chained_if(ctas_of(grid) <= (under_capture(s) ? 64u : 132u), dft_gather_kernel<float>, grid, dim3(256), 0, s,
+                      regions, total_pts, reinterpret_cast<const float* const*>(fields), ny, pitch,
+                      static_cast<long long>(slot), static_cast<float*>(buf));
   return 1;
 }
 

@@ -7,6 +7,7 @@
 // only what it copied itself, so no CTA barrier is needed) and runs the same
 // update as the other sweeps (fused3d_common.cuh).
 #include <algorithm>
+#include <cmath>
 
 #include "fused3d_common.cuh"
 
@@ -206,19 +207,37 @@ static int carveout_for(int ctas, size_t smem) {
   return static_cast<int>(std::min<size_t>(100, (need * 100 + max_sm - 1) / max_sm));
 }
 
-// Whether to count a plane's groups along its rows instead of taking tiles of
-// 128 cells of 4 rows: where a tenth or more of the 128-cell tiles' groups
-// would lie beyond the rows' ends (nx = 132: 31 of 64). The division that
-// finds a group's row costs the full rows about 1%.
-static bool rows_padded(const FusedArgs& a) { return (a.nx + 3) / 4 * 10 <= a.pitch / 4 * 9; }
-
-static dim3 sweep_grid(const FusedArgs& a) {
+// The CTAs of a sweep, and whether to count a plane's groups along its rows
+// instead of taking tiles of 128 cells of 4 rows: where a tenth or more of the
+// 128-cell tiles' groups would lie beyond the rows' ends (nx = 132: 31 of 64), and
+// this saves the chip (`ctas` CTAs on each SM) part of a round of CTAs. Finding
+// a group's row costs large sweeps about 1%, but one round 8 to 20% (82 x 48 x 64,
+// 744 tiles on 1036 places or 496 CTAs along the rows: 9.24 and 10.7 us a step; 100
+// x 100 x 40, 950 or 760: 11.1 and 12.1); 70 x 79 x 55, 1060 or 583: 12.6 and 9.7.
+struct SweepGrid {
+  dim3 grid;
+  bool lin;
+};
+static SweepGrid sweep_grid(const FusedArgs& a, int ctas) {
   const unsigned planes = a.kend - a.kbeg;
-  if (rows_padded(a)) {
-    const long long groups = static_cast<long long>((a.nx + 3) / 4) * (a.ny - 2);
-    return dim3(static_cast<unsigned>((groups + kThreads - 1) / kThreads), 1, planes);
-  }
-  return dim3(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, planes);
+  const long long groups = static_cast<long long>((a.nx + 3) / 4) * (a.ny - 2);
+  const dim3 tiles(a.pitch / 128, (a.ny - 2 + kRowsA - 1) / kRowsA, planes);
+  const dim3 lin(static_cast<unsigned>((groups + kThreads - 1) / kThreads), 1, planes);
+  if ((a.nx + 3) / 4 * 10 > a.pitch / 4 * 9) return {tiles, false};
+  // rounds of CTAs; the last, part empty, takes between its share and a whole one
+  const double places = static_cast<double>(sm_count()) * ctas, rt = ctas_of(tiles) / places, rl = ctas_of(lin) / places;
+  auto time = [](double r) { return r <= 1.0 ? 1.0 : 0.5 * (r + std::ceil(r)); };
+  const bool less = rt <= 1.0 ? rt > 0.85 && rl <= 0.6 * rt : time(rl) * (1.0 + 0.15 / rt) < time(rt);
+  return {less ? lin : tiles, less};
+}
+
+// Whether a sweep's launch is chained. In a graph a sweep of one round of CTAs
+// behind another is not: 98 x 60 x 45, 645 CTAs: 10.8 us a step chained, 9.0 not;
+// 200 x 60 x 60, 1334: 15.5 and 16.2. Behind the small kernels of TFSF planes it
+// is (70 x 79 x 55 with a box: 24.9 and 26.2).
+static bool sweep_chains(const FusedArgs& a, dim3 grid, cudaStream_t s) {
+  if (!chains(grid)) return false;
+  return a.nplanes > 0 || ctas_of(grid) > 7ull * sm_count() || !under_capture(s);
 }
 
 // CTAs per SM: 7 (6 for two poles) with the ADE state read per component;
@@ -229,16 +248,17 @@ static void staged_e_launch(const FusedArgs& a, cudaStream_t s) {
   constexpr int slots = kSlotsE + (PJ ? pj_slots<MAXP>() : 0);
   constexpr int minb = !PJ ? (MAXP >= 2 ? 6 : 7) : (MAXP >= 2 ? 4 : (MAXP == 1 ? 6 : 7));
   const size_t smem = slots * kThreads * sizeof(float4) + kThreads * sizeof(unsigned);
+  const SweepGrid g = sweep_grid(a, minb);
+  const bool chain = sweep_chains(a, g.grid, s);
   auto go = [&](auto fn) {
     // once per device: the shared-memory split that holds minb CTAs, the rest as L1
     once_per_device(reinterpret_cast<const void*>(fn), [&] {
       cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(minb, smem));
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     });
-    launch_chained(fn, sweep_grid(a), block, smem, s, a);
+    launch_chained_if(chain, fn, g.grid, block, smem, s, a);
   };
-  const bool chain = chains(sweep_grid(a));
-  if (rows_padded(a)) chain ? go(staged_e_kernel<MAXP, minb, PJ, true, true>) : go(staged_e_kernel<MAXP, minb, PJ, true, false>);
+  if (g.lin) chain ? go(staged_e_kernel<MAXP, minb, PJ, true, true>) : go(staged_e_kernel<MAXP, minb, PJ, true, false>);
   else chain ? go(staged_e_kernel<MAXP, minb, PJ, false, true>) : go(staged_e_kernel<MAXP, minb, PJ, false, false>);
 }
 
@@ -267,14 +287,15 @@ template <bool MU>
 static void staged_h_dispatch(const FusedArgs& a, cudaStream_t s) {
   const dim3 block(32, kRowsA, 1);
   const size_t smem = kSlotsH * kThreads * sizeof(float4);
+  const SweepGrid g = sweep_grid(a, 8);
+  const bool chain = sweep_chains(a, g.grid, s);
   auto go = [&](auto fn) {
     once_per_device(reinterpret_cast<const void*>(fn), [&] {
       cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_for(8, smem));
     });
-    launch_chained(fn, sweep_grid(a), block, smem, s, a);
+    launch_chained_if(chain, fn, g.grid, block, smem, s, a);
   };
-  const bool chain = chains(sweep_grid(a));
-  if (rows_padded(a)) chain ? go(staged_h_kernel<8, MU, true, true>) : go(staged_h_kernel<8, MU, true, false>);
+  if (g.lin) chain ? go(staged_h_kernel<8, MU, true, true>) : go(staged_h_kernel<8, MU, true, false>);
   else chain ? go(staged_h_kernel<8, MU, false, true>) : go(staged_h_kernel<8, MU, false, false>);
 }
 

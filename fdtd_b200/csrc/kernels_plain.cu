@@ -776,14 +776,33 @@ static int plain_carveout(size_t smem, int ctas) {
 }
 
 template <class F>
-static void plain_launch(F fn, size_t smem, const dim3& grid, const dim3& block, const PlainArgs& a,
+static void plain_launch(F fn, size_t smem, const dim3& grid, const dim3& block, const PlainArgs& a, bool chain,
                          cudaStream_t s) {
   const int ctas = block.x * block.y == 256 ? 2 : 3;
   once_per_device(reinterpret_cast<const void*>(fn), [&] {
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, plain_carveout(smem, ctas));
   });
-  launch_chained(fn, grid, block, smem, s, a);
+  launch_chained_if(chain, fn, grid, block, smem, s, a);
+}
+
+// Whether the FP64 sweeps are chained: all 2D ones and those launched one by one; of
+// 3D grids in a graph those of one and a half rounds of CTAs (two on each SM) or
+// more, of one round with TFSF planes, and those with cells without poles that leave
+// three quarters of the places free (half, where nothing comes between them). Between
+// these a chained sweep's CTAs find places beside some of the last one's only: us a
+// step chained and not, 0.17 rounds (36^3) 32.9 and 33.6, 0.41 (130 x 42 x 50) with a
+// pole everywhere 52.9 and 42.6, 0.88 (100 x 100 x 40) 42.1 and 39.3, 1.08 (132 x 64 x
+// 60) 43.5 and 39.8, 1.51 (200 x 60 x 60) 62.9 and 63.3, 6.9 (173 x 150 x 141) 209.1 and
+// 210.8; with a TFSF box 0.49 (82 x 48 x 64) 55.4 and 50.1, 1.08 57.5 and 59.4. (Not
+// all: 0.65 rounds, 124 x 50 x 60 gains 10% by the chain, 98 x 90 x 50 loses 6%.)
+template <int MODE>
+static bool plain_chains(const PlainArgs& a, dim3 h, cudaStream_t s) {
+  if (!chains(h)) return false;
+  if (MODE != kThreeD || !under_capture(s)) return true;
+  const double rounds = ctas_of(h) / (2.0 * sm_count());
+  if (rounds >= (a.nplanes > 0 ? 1.0 : 1.5)) return true;
+  return rounds <= (a.nplanes + a.gathers > 0 ? 0.25 : 0.5) && !a.all_dispersive;
 }
 
 // ZC planes per thread along z (3D): the copies of plane z + 1 go into the
@@ -806,17 +825,18 @@ static int launch_plain(const PlainArgs& a, cudaStream_t s, bool e) {
   };
   constexpr int T = kPlainThreads;
   const dim3 block(32, T / 32, 1), block2(32, T2 / 32, 1);
+  const bool chain = plain_chains<MODE>(a, grid(a.bd ? 1 : ZP, T), s);
   if (!e) {
-    if (a.bd) plain_launch(plain_h_kernel<MODE, true, 1, T>, bytes(1, 0, 1, T), grid(1, T), block, a, s);
-    else plain_launch(plain_h_kernel<MODE, false, ZP, T>, bytes(1, 0, ZP, T), grid(ZP, T), block, a, s);
+    if (a.bd) plain_launch(plain_h_kernel<MODE, true, 1, T>, bytes(1, 0, 1, T), grid(1, T), block, a, chain, s);
+    else plain_launch(plain_h_kernel<MODE, false, ZP, T>, bytes(1, 0, ZP, T), grid(ZP, T), block, a, chain, s);
   } else if (a.bd) {
-    plain_launch(plain_e_kernel<MODE, 0, true, 1, T>, bytes(0, 0, 1, T), grid(1, T), block, a, s);
+    plain_launch(plain_e_kernel<MODE, 0, true, 1, T>, bytes(0, 0, 1, T), grid(1, T), block, a, chain, s);
   } else if (a.all_dispersive && a.dispersive == 1) {
-    plain_launch(plain_e_kernel<MODE, 1, false, ZP, T>, bytes(0, 1, ZP, T), grid(ZP, T), block, a, s);
+    plain_launch(plain_e_kernel<MODE, 1, false, ZP, T>, bytes(0, 1, ZP, T), grid(ZP, T), block, a, chain, s);
   } else if (a.all_dispersive && a.dispersive == 2) {
-    plain_launch(plain_e_kernel<MODE, 2, false, ZP, T2>, bytes(0, 2, ZP, T2), grid(ZP, T2), block2, a, s);
+    plain_launch(plain_e_kernel<MODE, 2, false, ZP, T2>, bytes(0, 2, ZP, T2), grid(ZP, T2), block2, a, chain, s);
   } else {
-    plain_launch(plain_e_kernel<MODE, 0, false, ZP, T>, bytes(0, 0, ZP, T), grid(ZP, T), block, a, s);
+    plain_launch(plain_e_kernel<MODE, 0, false, ZP, T>, bytes(0, 0, ZP, T), grid(ZP, T), block, a, chain, s);
   }
   return 1;
 }
