@@ -748,7 +748,7 @@ PlainArgs plain_args(fdtd_grid* g) {
   a.tfsf_pre = g->d_tfsf_pre;
   a.tfsf_cells = g->tfsf_cells;
   a.dispersive = g->max_poles;
-  a.gathers = (g->ndft[0] > 0) + (g->ndft[1] > 0);
+  a.between = (g->ndft[0] > 0) + (g->ndft[1] > 0) + (g->bcs.n > 0);
   a.all_dispersive = g->mats.empty() ? 0 : 1;
   for (auto& m : g->mats)
     if (m.kind != FDTD_DRUDE && m.kind != FDTD_LORENTZ) a.all_dispersive = 0;

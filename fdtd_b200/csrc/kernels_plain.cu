@@ -802,7 +802,7 @@ static bool plain_chains(const PlainArgs& a, dim3 h, cudaStream_t s) {
   if (MODE != kThreeD || !under_capture(s)) return true;
   const double rounds = ctas_of(h) / (2.0 * sm_count());
   if (rounds >= (a.nplanes > 0 ? 1.0 : 1.5)) return true;
-  return rounds <= (a.nplanes + a.gathers > 0 ? 0.25 : 0.5) && !a.all_dispersive;
+  return rounds <= (a.nplanes + a.between > 0 ? 0.25 : 0.5) && !a.all_dispersive;
 }
 
 // ZC planes per thread along z (3D): the copies of plane z + 1 go into the

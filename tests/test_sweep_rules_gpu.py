@@ -58,7 +58,7 @@ def test_groups_along_rows_of_more_than_a_round(fdtd, nx, ny, nz):
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
-@pytest.mark.parametrize("kind", ["plain", "box", "dft", "box-dft", "poles"])
+@pytest.mark.parametrize("kind", ["plain", "box", "dft", "box-dft", "poles", "periodic-dft"])
 @pytest.mark.parametrize("nx,ny,nz", [(36, 36, 36), (60, 60, 40), (70, 79, 55), (98, 150, 45), (130, 120, 90)])
 def test_replayed_steps_equal_launched_ones(fdtd, prec, kind, nx, ny, nz):
     p = _problem(nx, ny, nz, "box" in kind, kind == "poles", "dft" in kind)
@@ -66,6 +66,10 @@ def test_replayed_steps_equal_launched_ones(fdtd, prec, kind, nx, ny, nz):
     for graphs in (True, False):
         g = fdtd.Grid.from_problem(p, prec)
         g.use_graphs(graphs)
+        if "periodic" in kind:
+            for a in range(3):
+                for s in (0, 1):
+                    g.set_boundary(a, s, "periodic")
         g.step(64)
         g.step(64)
         out.append([g.get(n) for n in NAMES] + [g.dft(h) for h in g.dft_handles])
