@@ -786,22 +786,26 @@ static void plain_launch(F fn, size_t smem, const dim3& grid, const dim3& block,
   launch_chained_if(chain, fn, grid, block, smem, s, a);
 }
 
-// Whether the FP64 sweeps are chained: all 2D ones and those launched one by one; of
-// 3D grids in a graph those of one and a half rounds of CTAs (two on each SM) or
+// Whether the FP64 sweeps are chained: all 2D ones, nearly all launched one by one; of
+// 3D grids in a graph those of one and a quarter rounds of CTAs (two on each SM) or
 // more, of one round with TFSF planes, and those with cells without poles that leave
 // three quarters of the places free (half, where nothing comes between them). Between
 // these a chained sweep's CTAs find places beside some of the last one's only: us a
 // step chained and not, 0.17 rounds (36^3) 32.9 and 33.6, 0.41 (130 x 42 x 50) with a
 // pole everywhere 52.9 and 42.6, 0.88 (100 x 100 x 40) 42.1 and 39.3, 1.08 (132 x 64 x
-// 60) 43.5 and 39.8, 1.51 (200 x 60 x 60) 62.9 and 63.3, 6.9 (173 x 150 x 141) 209.1 and
-// 210.8; with a TFSF box 0.49 (82 x 48 x 64) 55.4 and 50.1, 1.08 57.5 and 59.4. (Not
-// all: 0.65 rounds, 124 x 50 x 60 gains 10% by the chain, 98 x 90 x 50 loses 6%.)
+// 60) 43.5 and 39.8, 1.32 (173 x 42 x 103) 72.7 and 73.8, 1.51 (200 x 60 x 60) 62.9
+// and 63.3, 6.9 (173 x 150 x 141) 209.1 and 210.8; with a TFSF box 0.49 (82 x 48 x 64)
+// 55.4 and 50.1, 1.08 57.5 and 59.4. (Not all: at 0.65 rounds 124 x 50 x 60 gains 10%
+// by the chain, at 0.67 98 x 90 x 50 loses 6%.)
 template <int MODE>
 static bool plain_chains(const PlainArgs& a, dim3 h, cudaStream_t s) {
   if (!chains(h)) return false;
-  if (MODE != kThreeD || !under_capture(s)) return true;
+  if (MODE != kThreeD) return true;
   const double rounds = ctas_of(h) / (2.0 * sm_count());
-  if (rounds >= (a.nplanes > 0 ? 1.0 : 1.5)) return true;
+  // (one by one, two poles everywhere: 0.49 rounds, 82 x 48 x 64, 44.5 and 42.2; 0.2, 50 x
+  // 40 x 44, 39.7 and 41.4; 0.65, 124 x 50 x 60, 52.8 and 54.2)
+  if (!under_capture(s)) return !(a.all_dispersive && a.dispersive == 2 && rounds > 0.25 && rounds < 0.6);
+  if (rounds >= (a.nplanes > 0 ? 1.0 : 1.25)) return true;
   return rounds <= (a.nplanes + a.between > 0 ? 0.25 : 0.5) && !a.all_dispersive;
 }
 
